@@ -24,6 +24,7 @@
 #include "kernels_band.cuh"
 #include "kernels_multi.cuh"
 #include "kernels_exact.cuh"
+#include "kernels_resident.cuh"
 
 using namespace swit;
 
@@ -55,6 +56,8 @@ namespace swit {
 // Lets other translation units of the library report through swit_last_error.
 void set_last_error(const char* msg) { g_err = msg; }
 }  // namespace swit
+
+struct ResLoop;
 
 constexpr int kCapStreamsMax = 4;  // concurrent branches of a captured graph, at most
 
@@ -137,6 +140,9 @@ struct swit_engine {
   void *xm = nullptr, *xsrc = nullptr, *xdadc = nullptr;
   std::vector<cudaGraphExec_t> gxb;
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
+  // resident time loops (kernels_resident.cuh), where the split fits the device; else the variant's kernels
+  ResLoop *resf = nullptr, *resb = nullptr;
+  uint4* d_halo = nullptr;
 };
 
 namespace {
@@ -164,6 +170,8 @@ int valloc(swit_engine* e, void** ptr, size_t n) {
   return 0;
 }
 
+void res_free(swit_engine* e);
+
 void release(swit_engine* e) {
   for (auto* v : {&e->gfwd[0], &e->gfwd[1], &e->gbwd, &e->gxb}) {
     for (cudaGraphExec_t x : *v) cudaGraphExecDestroy(x);
@@ -182,9 +190,10 @@ void release(swit_engine* e) {
                   e->d_mtrace, e->A, e->B, e->damp, e->cint, e->kp, e->ku, e->kw, e->p, e->u, e->w, e->pb, e->ub, e->wb, e->pe,
                   e->ue, e->we, e->dg, e->dfw, e->dbk, e->strips, e->src, e->seis_t, e->adj_t, e->d_in, e->d_src_in,
                   e->d_stage, e->p2, e->u2, e->w2, e->pb2, e->ub2, e->wb2, e->pe2, e->ue2, e->we2, e->d_list, e->d_dlist, e->d_blist, e->d_bcnt, e->d_err, e->ckpt,
-                  e->xm, e->xsrc, e->xdadc};
+                  e->xm, e->xsrc, e->xdadc, e->d_halo};
   for (void* q : ptrs)
     if (q) cudaFree(q);
+  res_free(e);
 }
 
 template <class R>
@@ -224,6 +233,16 @@ inline Receivers make_rec(const swit_engine* e) {
   return Receivers{e->d_colptr, e->d_ig, e->d_zr, e->d_zlo, e->d_zhi, e->rcomp, e->d_rcol};
 }
 inline Sources make_src(const swit_engine* e) { return Sources{e->d_isx, e->d_isz, e->d_risx, e->d_risz}; }
+
+}  // namespace
+#include "resident_host.cuh"
+namespace {
+
+void res_free(swit_engine* e) {
+  delete e->resf;
+  delete e->resb;
+  e->resf = e->resb = nullptr;
+}
 
 // Launch shape of the stencil kernels for a batch of nb shots.
 inline void stencil_shape(const swit_engine* e, int nb, dim3& grid, dim3& block) {
@@ -344,8 +363,12 @@ void launch_bwd_walk(swit_engine* e, int shot0, int nb, int it, cudaStream_t st)
 // Forward time loop of shots [shot0, shot0+nb): fdcore.f90:75-160.
 template <class R>
 void launch_forward_steps(swit_engine* e, bool store, int shot0, int nb, cudaStream_t st, int it_lo = 2,
-                          int it_hi = -1) {
+                          int it_hi = -1, bool res = false) {
   if (it_hi < 0) it_hi = e->nt;
+  if (res) {
+    res_forward(e, *e->resf, store, shot0, nb, st, it_lo, it_hi);
+    return;
+  }
   if (e->variant == 4 || e->variant == 5) {
     if (e->maxt_f == 512)
       launch_cluster_fwd_t<R, 512>(e, store, shot0, nb, st);
@@ -402,7 +425,8 @@ void launch_forward_steps(swit_engine* e, bool store, int shot0, int nb, cudaStr
 
 // Reverse time loop of shots [shot0, shot0+nb): solver.f90:230-253.
 template <class R>
-void launch_backward_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int it_hi = -1, int it_lo = 2) {
+void launch_backward_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int it_hi = -1, int it_lo = 2,
+                           bool res = false) {
   if (it_hi < 0) it_hi = e->nt;
   if (e->variant == 4) {
     if (e->maxt_b == 512)
@@ -483,10 +507,10 @@ inline void ckpt_copy(swit_engine* e, int slot, int s0, int nb, bool save, int i
 
 // Forward of shots [s0, s0+nb) keeping checkpoints instead of strips.
 template <class R>
-void forward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st) {
+void forward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st, bool res = false) {
   const int k = e->ckpt_k;
   for (int m = 0; m < e->ckpt_m; ++m) {
-    launch_forward_steps<R>(e, false, s0, nb, st, std::max(2, m * k + 1), std::min(e->nt, (m + 1) * k));
+    launch_forward_steps<R>(e, false, s0, nb, st, std::max(2, m * k + 1), std::min(e->nt, (m + 1) * k), res);
     ckpt_copy(e, m, s0, nb, true, std::min(e->nt, (m + 1) * k), st);
   }
 }
@@ -496,7 +520,7 @@ void forward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st) {
 // (the same kernels, so the same strips as a boundary-saving run), then run
 // the reverse steps that read them.  Leaves sit0 = 1.
 template <class R>
-void backward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st) {
+void backward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st, bool res = false) {
   const int k = e->ckpt_k;
   const size_t fsz = (size_t)e->NX * e->LD * e->esz;
   for (int m = e->ckpt_m - 1; m >= 0; --m) {
@@ -512,8 +536,8 @@ void backward_checkpointed(swit_engine* e, int s0, int nb, cudaStream_t st) {
                       (size_t)nb * e->snt * e->SL * e->esz, st);
     }
     e->sit0 = m * k + 1;
-    launch_forward_steps<R>(e, true, s0, nb, st, std::max(2, m * k + 1), std::min(e->nt, (m + 1) * k));
-    launch_backward_steps<R>(e, s0, nb, st, std::min(e->nt, (m + 1) * k + 1), m * k + 2);
+    launch_forward_steps<R>(e, true, s0, nb, st, std::max(2, m * k + 1), std::min(e->nt, (m + 1) * k), res);
+    launch_backward_steps<R>(e, s0, nb, st, std::min(e->nt, (m + 1) * k + 1), m * k + 2, res);
   }
   e->sit0 = 1;
 }
@@ -686,6 +710,14 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
       else
         launch_forward_steps<R>(e, store, s, 1, st);
     }
+    CK(cudaGetLastError());
+    return 0;
+  }
+  if (e->resf && !(store && e->exact && !e->ckpt_k)) {  // the storing exact forward keeps D of every step
+    if (store && e->ckpt_k)
+      forward_checkpointed<R>(e, 0, e->ns, st, true);
+    else
+      launch_forward_steps<R>(e, store, 0, e->ns, st, 2, e->nt, true);
     CK(cudaGetLastError());
     return 0;
   }
@@ -974,8 +1006,11 @@ int residual_l2(swit_engine* e, const float* obs, int on_device, cudaStream_t st
 // Sum of the per-trace misfits on the host (waits for the stream).
 int misfit_sum(swit_engine* e, cudaStream_t st, double* misfit) {
   std::vector<double> mt((size_t)e->ns * e->ngmax);
+  int err = 0;
   CK(cudaMemcpyAsync(mt.data(), e->d_mtrace, mt.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (e->resf) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (err) return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
   double acc = 0.0;
   for (double v : mt) acc += v;
   *misfit = acc;
@@ -1996,6 +2031,37 @@ void auto_batches(swit_engine* e, int branches) {
   e->branches = br;
 }
 
+// Resident time loops for FP32 engines on the default kernels and launch
+// shapes, where a split fits the device.  A checkpointed engine runs both loops
+// segment by segment over all shots, so it takes them only together and for
+// segments long enough to pay for loading and storing the state; vx adjoint
+// sources change u between the phases, also in the columns a band recomputes,
+// which the resident reverse loop does not do.
+static int res_setup(swit_engine* e, const swit_desc* d) {
+  if (d->kernel_variant || e->prec || e->path || d->shots_per_batch || d->graph_branches || d->block_x) return 0;
+  if (const char* v = std::getenv("SWIT_RESIDENT"))
+    if (std::atoi(v) == 0) return 0;
+  if (e->ckpt_k && e->ckpt_k < 32) return 0;
+  ResLoop f, b;
+  res_choose(e, false, f);
+  if (!e->exact && e->rcomp != 1) res_choose(e, true, b);
+  if (e->ckpt_k && !e->exact && !(f.ok && b.ok)) return 0;
+  const size_t n = std::max(res_halo_packets(f), res_halo_packets(b));
+  if (!n) return 0;
+  if (int rc = dalloc(e, &e->d_halo, n)) return rc;
+  unsigned wait = kResWaitLimit;
+  if (const char* v = std::getenv("SWIT_RES_WAIT_POLLS")) {  // a shorter wait, e.g. to test the timeout path
+    const long long w = std::atoll(v);
+    if (w >= 0 && w < (long long)kResWaitLimit) wait = (unsigned)w;
+  }
+  f.r.halo = b.r.halo = e->d_halo;
+  f.r.err = b.r.err = e->d_err;
+  f.r.wait = b.r.wait = wait;
+  if (f.ok) e->resf = new ResLoop(f);
+  if (b.ok) e->resb = new ResLoop(b);
+  return 0;
+}
+
 int swit_create(const swit_desc* d, swit_engine** out) {
   if (!d || !out) return fail(SWIT_E_ARG, "null argument");
   *out = nullptr;
@@ -2286,6 +2352,12 @@ int swit_create(const swit_desc* d, swit_engine** out) {
       return rc;
     }
   }
+  rc = res_setup(e, d);
+  if (rc) {
+    release(e);
+    delete e;
+    return rc;
+  }
   // Entries never written by the kernels must read as zero: step 1 of the
   // seismograms (fdcore.f90 starts at it = 2), traces beyond ng(is), and the
   // strips of step 1 that the reconstruction inserts at it = 2.
@@ -2314,7 +2386,21 @@ int swit_create(const swit_desc* d, swit_engine** out) {
   const int fwaves = e->path == 1 ? ns : (ns + fwd_batch(e) - 1) / fwd_batch(e);
   e->launches_fwd = (e->variant == 4 || e->variant == 5) ? fwaves : per * (e->nt - 1) * per_step;
   e->launches_bwd = e->variant == 4 ? per : per * (e->nt - 1) * per_step * (e->ckpt_k ? 2 : 1);
+  const int segs = std::max(1, e->ckpt_m);
+  const int resf = e->resf ? segs * ((ns + e->resf->shots - 1) / e->resf->shots) : 0;
+  if (e->resf && !(e->exact && !e->ckpt_k)) e->launches_fwd = resf;
+  if (e->resb)
+    e->launches_bwd = segs * ((ns + e->resb->shots - 1) / e->resb->shots) + (e->ckpt_k ? resf : 0);
   *out = e;
+  return 0;
+}
+
+// End of a call with host buffers: waits for the stream; the resident loops report a wait that gave up.
+static int host_end(swit_engine* e, cudaStream_t st) {
+  int err = 0;
+  if (e->resf) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (err) return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
   return 0;
 }
 
@@ -2342,8 +2428,7 @@ int swit_forward(swit_engine* e, const float* src, void* seis, int save_boundary
   int rc = e->prec ? forward_impl<double>(e, src, seis, save_boundary != 0, on_device, st)
                    : forward_impl<float>(e, src, seis, save_boundary != 0, on_device, st);
   if (rc) return rc;
-  if (!on_device) CK(cudaStreamSynchronize(st));
-  return 0;
+  return on_device ? 0 : host_end(e, st);
 }
 
 int swit_backward(swit_engine* e, const float* adj, void* grad, void* illum_fw, void* illum_bk, int on_device,
@@ -2355,8 +2440,7 @@ int swit_backward(swit_engine* e, const float* adj, void* grad, void* illum_fw, 
   int rc = e->prec ? backward_impl<double>(e, adj, grad, illum_fw, illum_bk, on_device, st)
                    : backward_impl<float>(e, adj, grad, illum_fw, illum_bk, on_device, st);
   if (rc) return rc;
-  if (!on_device) CK(cudaStreamSynchronize(st));
-  return 0;
+  return on_device ? 0 : host_end(e, st);
 }
 
 int swit_gradient_l2(swit_engine* e, const float* src, const float* obs, void* grad, void* illum_fw, void* illum_bk,
@@ -2467,7 +2551,7 @@ int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_b
   if (block_x) *block_x = e->bx;
   if (kernels_per_forward) *kernels_per_forward = e->launches_fwd;
   if (kernels_per_backward) *kernels_per_backward = e->launches_bwd;
-  if (kernel_variant) *kernel_variant = e->variant;
+  if (kernel_variant) *kernel_variant = e->resf && e->resb ? 7 : e->variant;
   return 0;
 }
 
@@ -2478,7 +2562,7 @@ int swit_check(swit_engine* e, void* stream) {
   CK(cudaMemcpy(&w, e->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (w) {
     CK(cudaMemset(e->d_err, 0, sizeof(int)));
-    return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting for its staged copies (error word %d); results are invalid", w);
+    return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting for its copies or a neighbour's halo (error word %d); results are invalid", w);
   }
   return 0;
 }

@@ -228,7 +228,7 @@ class Engine:
         kind = self.query()["kernel"]
         if kind == "walk":
             names = ("fwd_step", None, "bwd_step", None)
-        elif kind == "cluster":
+        elif kind in ("cluster", "resident"):
             names = ("fwd_loop", None, "bwd_loop", None)
         elif kind == "hybrid":
             names = ("fwd_loop", None, "bwd_uw", "bwd_p")
@@ -241,7 +241,8 @@ class Engine:
                                         C.byref(kv), C.byref(br)))
         return dict(device_bytes=by.value, shots_per_batch=sb.value, block_x=bx.value, graph_branches=br.value,
                     kernels_per_forward=kf.value,
-                    kernels_per_backward=kb.value, kernel={1: "split", 2: "walk", 3: "vec", 4: "cluster", 5: "hybrid", 6: "band"}.get(kv.value, "?"))
+                    kernels_per_backward=kb.value, kernel={1: "split", 2: "walk", 3: "vec", 4: "cluster", 5: "hybrid", 6: "band",
+                            7: "resident"}.get(kv.value, "?"))
 
     def check(self):
         """Waits for torch's current stream and raises SwitError if a kernel gave

@@ -1,0 +1,87 @@
+"""Resident time loops (csrc/kernels_resident.cuh): the default kernels of FP32
+engines, against the FP32 oracle.
+
+The loops evaluate the oracle's expressions in its order without FMA, so every
+result is expected bit for bit: seismograms, strips, end states, gradient and
+illuminations.  The sizes sit where a split can go wrong: bands of one, two and
+three 4-column tiles and a shot in one band, grids whose last tile has 1 to 4
+columns, every alignment of the free surface and of the bottom row to the 4-row
+tiles, the smallest grid, columns of several warps, scattered and coinciding
+receivers.  SWIT_RES_FWD_TILES / SWIT_RES_BWD_TILES set the band width.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from swit_gb300 import Engine, SwitError, survey
+
+pytestmark = pytest.mark.gpu
+
+
+def problem(nx=37, nz=28, npml=9, nt=140, ns=2, zs=20.0, zr=10.0, free_surface=1, comp="p", scattered=False):
+    s = survey.small(nx=nx, nz=nz, npml=npml, nt=nt, ns=ns, zs=zs, zr=zr)
+    s.free_surface = free_surface
+    if scattered:  # two nodes with several receivers, one receiver off the line
+        rec = s.rec_xz.copy()
+        rec[:, 5] = rec[:, 4] + np.array([3.0, 0.0], np.float32)
+        rec[:, 9] = rec[:, 4]
+        rec[:, 7, 1] += 20.0
+        s.rec_xz = rec
+    pb = O.Problem(s.nx, s.nz, s.npml, s.nt, s.dx, s.dt, s.src_xz, s.rec_xz, free_surface=free_surface, comp=comp)
+    return s, pb
+
+
+def split(monkeypatch, tiles):
+    for k in ("SWIT_RES_FWD_TILES", "SWIT_RES_BWD_TILES"):
+        monkeypatch.setenv(k, str(tiles))
+
+
+SHAPES = ([(dict(nx=37, nz=28, npml=n), t) for n in (8, 9, 10, 11) for t in (1, 2)] +
+          [(dict(nx=nx, nz=30, npml=7), 3) for nx in (34, 35, 36, 37)] +
+          [(dict(nx=36, nz=nz, npml=8, zs=70.0, zr=0.0), 2) for nz in (27, 28, 29, 30)] +
+          [(dict(nx=8, nz=8, npml=2, ns=1, nt=60), 3), (dict(nx=8, nz=8, npml=2, ns=1, nt=60), 1),
+           (dict(nx=40, nz=36, npml=8, zs=120.0, free_surface=0), 2), (dict(nx=40, nz=36, npml=9, scattered=True), 15),
+           (dict(nx=40, nz=36, npml=9, zr=60.0, zs=120.0, scattered=True), 1), (dict(nx=61, nz=210, npml=12, nt=90), 2),
+           (dict(comp="vx"), 2), (dict(comp="vz"), 2)])
+
+
+@pytest.mark.parametrize("shape,tiles", SHAPES)
+def test_forward_matches_oracle(shape, tiles, monkeypatch):
+    s, pb = problem(**shape)
+    src, rho = s.source(), s.rho(s.vp_true)
+    ref = O.forward(pb, s.vp_true, rho, src, store=True)
+    split(monkeypatch, tiles)
+    with Engine(**s.engine_args(), receiver_component=shape.get("comp", "p")) as e:
+        e.set_model(s.vp_true, rho)
+        plain = e.forward(src, save_boundary=False)
+        seis = e.forward(src, save_boundary=True)
+        snap = e.export_snapshot()
+        e.check()
+    np.testing.assert_array_equal(seis, ref["seis"])
+    np.testing.assert_array_equal(plain, ref["seis"])
+    for k in ("boundary", "p_end", "u_end", "w_end"):
+        np.testing.assert_array_equal(snap[k], ref[k], err_msg=k)
+
+
+def test_halo_timeout_is_reported_and_the_context_stays_usable(monkeypatch):
+    """With a poll limit of 0 every halo wait gives up at its first miss, records
+    it in the engine's error word and goes on without waiting: the call with host
+    buffers raises, check() clears the word, and an engine created afterwards
+    computes the oracle's seismograms."""
+    s, pb = problem()
+    src, rho = s.source(), s.rho(s.vp_true)
+    ref = O.forward(pb, s.vp_true, rho, src, store=False)
+    split(monkeypatch, 1)
+    monkeypatch.setenv("SWIT_RES_WAIT_POLLS", "0")
+    with Engine(**s.engine_args()) as e:
+        e.set_model(s.vp_true, rho)
+        with pytest.raises(SwitError, match="SWIT_E_TIMEOUT"):
+            e.forward(src, save_boundary=False)
+        with pytest.raises(SwitError, match="SWIT_E_TIMEOUT"):
+            e.check()
+        e.check()  # the word was cleared
+    monkeypatch.delenv("SWIT_RES_WAIT_POLLS")
+    with Engine(**s.engine_args()) as e:
+        e.set_model(s.vp_true, rho)
+        np.testing.assert_array_equal(e.forward(src, save_boundary=False), ref["seis"])
+        e.check()
