@@ -82,7 +82,11 @@ typedef struct swit_desc {
                                cluster kernels: CTAs per cluster 1..16 (default
                                16; the reverse loop takes more CTAs when its six
                                wavefields need them)                            */
-  int32_t kernel_variant;   /* 0 = automatic (vec), 1 = split: two kernels per step,
+  int32_t kernel_variant;   /* 0 = automatic: FP32 engines on the batched path with
+                               default launch shapes run whole time loops with
+                               the wavefields in registers where the shots fit
+                               the device (swit_query reports 7 when both loops
+                               do), else vec; 1 = split: two kernels per step,
                                in place, one point per thread; 2 = walk: one
                                kernel per step, double-buffered, each warp
                                walking a tile of columns with the x-neighbours

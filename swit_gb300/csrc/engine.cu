@@ -428,6 +428,10 @@ template <class R>
 void launch_backward_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int it_hi = -1, int it_lo = 2,
                            bool res = false) {
   if (it_hi < 0) it_hi = e->nt;
+  if (res) {
+    res_backward(e, *e->resb, shot0, nb, st, it_hi, it_lo);
+    return;
+  }
   if (e->variant == 4) {
     if (e->maxt_b == 512)
       launch_cluster_bwd_t<R, 512>(e, shot0, nb, st);
@@ -747,6 +751,14 @@ int run_backward_loop(swit_engine* e, cudaStream_t st) {
       else
         launch_backward_steps<R>(e, s, 1, st);
     }
+    CK(cudaGetLastError());
+    return 0;
+  }
+  if (e->resb) {
+    if (e->ckpt_k)
+      backward_checkpointed<R>(e, 0, e->ns, st, true);
+    else
+      launch_backward_steps<R>(e, 0, e->ns, st, e->nt, 2, true);
     CK(cudaGetLastError());
     return 0;
   }
@@ -1237,9 +1249,38 @@ int profile_vec_graphs(swit_engine* e, int32_t launches[4], double mean_ms[4], c
   return rc;
 }
 
+// Resident loops: events around every launch of one forward (launches[0], mean_ms[0]) and one reverse loop
+// ([2]) over all shots, from zero fields.
+int profile_resident(swit_engine* e, int32_t launches[4], double mean_ms[4], cudaStream_t st) {
+  const size_t fb = (size_t)e->ns * e->NX * e->LD * sizeof(float);
+  for (void* q : {e->p, e->u, e->w, e->pb, e->ub, e->wb, e->pe, e->ue, e->we, e->dg, e->dfw, e->dbk})
+    CK(cudaMemsetAsync(q, 0, fb, st));
+  std::vector<cudaEvent_t> ev[2];
+  res_forward(e, *e->resf, true, 0, e->ns, st, 2, e->nt, &ev[0]);
+  res_backward(e, *e->resb, 0, e->ns, st, e->nt, 2, &ev[1]);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(st));
+  for (int q = 0; q < 2; ++q) {
+    double tot = 0.0;
+    for (size_t i = 0; i + 1 < ev[q].size(); i += 2) {
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, ev[q][i], ev[q][i + 1]);
+      tot += ms;
+    }
+    launches[2 * q] = (int32_t)(ev[q].size() / 2);
+    mean_ms[2 * q] = tot / std::max<size_t>(ev[q].size() / 2, 1);
+    launches[2 * q + 1] = 0;
+    mean_ms[2 * q + 1] = 0.0;
+    for (cudaEvent_t x : ev[q]) cudaEventDestroy(x);
+  }
+  return 0;
+}
+
 template <class R>
 int profile_impl(swit_engine* e, int32_t launches[4], double mean_ms[4], cudaStream_t st) {
   if (e->ckpt_k) return fail(SWIT_E_STATE, "this call needs boundary saving (checkpoint_every = 0)");
+  if constexpr (sizeof(R) == 4)
+    if (e->resf && e->resb) return profile_resident(e, launches, mean_ms, st);
   if (e->variant == 3 && e->path == 0) return profile_vec_graphs<R>(e, launches, mean_ms, st);
   Grid<R> g = make_grid<R>(e);
   const int nshot_launch = e->path == 1 ? 1 : e->batch;

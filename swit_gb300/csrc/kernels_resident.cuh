@@ -908,4 +908,307 @@ __global__ void __launch_bounds__(MAXT, 1)
   tile_store<TX>(W_ + off, g.LD, T.ix0, iz0, live, 1, NZ, 1, NX, w);
 }
 
+// ---------------------------------------------------------------------------
+// What the reconstruction of a band re-inserts at one step (the strips of the
+// step before): per column {-, T0, T1, T2} and {B0, B1, B2, -}, and the six side
+// arrays of bands at (or next to) the sides (row jz at float jz); then the
+// step's adjoint sources.  Two boxes by step parity.
+__device__ __forceinline__ int box_at(const ResPlan& r, int it) { return r.oBox + (it & 1) * r.box; }
+__device__ __forceinline__ int strip_t(const ResPlan& r, int it) { return box_at(r, it); }
+__device__ __forceinline__ int strip_b(const ResPlan& r, int it) { return box_at(r, it) + r.W; }
+__device__ __forceinline__ int strip_s(const ResPlan& r, int it, int a) { return box_at(r, it) + 2 * r.W + a * r.nqr; }
+__device__ __forceinline__ int box_adj(const ResPlan& r, int it) { return box_at(r, it) + 2 * r.W + 6 * r.nqr; }
+// Replaces the rows of column f that lie on the interior by side array a.
+template <int TX>
+__device__ __forceinline__ void insert_row(bool on, int at, int k, float (&f)[TX][4], int j) {
+#pragma unroll
+  for (int c = 0; c < TX; c += 4) lds4x1_if(on, at + c, k, f[c][j], f[c + 1][j], f[c + 2][j], f[c + 3][j]);
+}
+// Row nz falls on the same row J of its tile in every column: a constant of the launch.
+#define SWIT_RES_ROW(j, call)                     \
+  if ((j) == 0) {                                 \
+    constexpr int J = 0;                          \
+    call;                                         \
+  } else if ((j) == 1) {                          \
+    constexpr int J = 1;                          \
+    call;                                         \
+  } else if ((j) == 2) {                          \
+    constexpr int J = 2;                          \
+    call;                                         \
+  } else {                                        \
+    constexpr int J = 3;                          \
+    call;                                         \
+  }
+template <int TX>
+__device__ __forceinline__ void side_insert(const Tile<TX>& T, const ResPlan& r, int it, int a, float (&f)[4]) {
+  float v[4];
+  lds4(strip_s(r, it, a) + opaque(T.k) - r.kr, v);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) f[j] = (T.f >> (kRows + j)) & 1u ? v[j] : f[j];
+}
+
+// Reverse loop, steps it1 .. it0 (solver.f90:230-253), of shots shot0 + block /
+// C: the first nA threads run the adjoint (fdcore.f90:293-375), the others the
+// reconstruction (fdcore.f90:202-289) on the same band, so each keeps three
+// fields and the sums of one side; the image needs one value per point from one
+// to the other, pb(t+1) - pb(t), through shared memory.
+//
+// Five 16-value arrays and the rest need more registers than 128: 384 threads of 168 are faster on a full
+// device than 512 of 128, which spill (49 shots 481x141: 3.1 against 4.4 us per step and launch, 13 and 10
+// launches).  Measured against the vec kernels: reverse loop of 49 shots 481x141, nt 1000: 59.8 -> 40.4 ms;
+// of 5 shots 201x101, nt 2000: 22.4 -> 5.7 ms.
+template <int TX, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_bwd_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,
+              const __grid_constant__ Sources src, const __grid_constant__ Receivers rec, const float* __restrict__ s_fwd,
+              const float* __restrict__ adj_t, float* __restrict__ PB, float* __restrict__ UB, float* __restrict__ WB,
+              float* __restrict__ PE, float* __restrict__ UE, float* __restrict__ WE, float* __restrict__ DG,
+              float* __restrict__ DFW, float* __restrict__ DBK, const float* __restrict__ strips, int it1, int it0,
+              int shot0) {
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int b = blockIdx.x % r.C, s = shot0 + blockIdx.x / r.C;
+  const int per = r.nt_tiles / r.C, rem = r.nt_tiles % r.C;
+  const int tt0 = b * per + min(b, rem), n = per + (b < rem ? 1 : 0);
+  const int fs = g.fs, L = g.L, NX = g.NX, NZ = g.NZ;
+  const float c1 = g.c1, c2 = g.c2;
+  // column tiles of the reconstruction in this band
+  const int q0 = max(tt0, r.m0), q1 = min(tt0 + n - 1, r.m1);
+  const int xoff = q0 - tt0, nr = q1 >= q0 ? q1 - q0 + 1 : 0;
+  int* s_cnt = reinterpret_cast<int*>(res_sm + r.oEnt);  // receiver entries
+  int* s_ig = s_cnt + 4;
+  int* s_code = s_ig + r.ent_cap;
+
+  for (int i = tid; i < r.smem / 16; i += nthr) res_sm[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  factor_setup(g, r, tt0 * TX + 1);
+  __syncthreads();
+  Tile<TX> T;
+  const bool adj0 = tid < r.nA;  // role, uniform over a warp
+  if (adj0)
+    tile_setup<TX, kResAdj>(T, g, r, tid, tt0, n, 0, r.nq, 0, b > 0, b < r.C - 1);
+  else
+    tile_setup<TX, kResRec>(T, g, r, tid - r.nA, q0, nr, xoff, r.nqr, r.kr, xoff == 0 && tt0 > r.m0,
+                            q1 == tt0 + n - 1 && q1 < r.m1);
+  float p[TX][4], u[TX][4], w[TX][4];
+  float s1[TX][4], s2[TX][4];  // adjoint: sum of pb^2, pb before the update; reconstruction: image, sum of pf^2
+  const size_t off = (size_t)s * g.FSZ;
+  unsigned gu;
+  RecTile R{0, 0, -1, 0};
+  int isrc = -1;  // source subtraction point, if it is in this tile
+  {
+    const int iz0 = row0<TX>(T, r, fs);
+    const bool live = T.f & kLive;
+    tile_load<TX>(adj0 ? g.A : g.B, g.LD, T.ix0, iz0, live, 1, NZ, 1, NX, p);
+    tile_load<TX>(adj0 ? g.B : g.A, g.LD, T.ix0, iz0, live, 1, NZ, 1, NX, u);
+#pragma unroll
+    for (int c = 0; c < TX; ++c) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        p[c][j] = adj0 ? p[c][j] : -p[c][j];
+        u[c][j] = adj0 ? u[c][j] : -u[c][j];
+      }
+      res_sm[r.oC + (2 * TX + 1) * tid + TX + c] = mk4(p[c]);
+      res_sm[r.oC + (2 * TX + 1) * tid + c] = mk4(u[c]);
+    }
+    const int z0 = adj0 ? 1 : L + 1, z1 = adj0 ? NZ : L + g.nz, x0 = adj0 ? 1 : L + 1, x1 = adj0 ? NX : L + g.nx;
+    tile_load<TX>((adj0 ? PB : PE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, p);
+    tile_load<TX>((adj0 ? UB : UE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, u);
+    tile_load<TX>((adj0 ? WB : WE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, w);
+    tile_load<TX>((adj0 ? DBK : DG) + off, g.LD, T.ix0, iz0, live, L + 1, L + g.nz, L + 1, L + g.nx, s1);
+    tile_load<TX>(DFW + off, g.LD, T.ix0, iz0, live && !adj0, L + 1, L + g.nz, L + 1, L + g.nx, s2);
+    if (adj0) {
+      gu = ghost_setup<TX, kResAdj>(T, g, r, UB + off);
+      R = rec_setup<TX>(T, g, r, rec, s, s_cnt, s_ig, s_code);
+      // one value per point goes to the reconstruction's tile in the same slot
+      const int xr = (T.ix0 - 1) / TX - q0, kq = T.k - r.kr;
+      const bool img = live && xr >= 0 && xr < nr && kq >= 0 && kq < r.nqr;
+      if (img) T.f |= kImg;
+      if (R.n > 0 && R.row < 0) T.f |= kRec;
+    } else {
+      gu = ghost_setup<TX, kResRec>(T, g, r, UE + off);
+      const int cx = src.risx[s] + L - T.ix0, jz = src.risz[s] + L - iz0;
+      if (live && src.risx[s] > 0 && cx >= 0 && cx < TX && jz >= 0 && jz < 4) isrc = 4 * cx + jz;
+    }
+  }
+  float snext = isrc >= 0 ? s_fwd[(size_t)s * (g.nt + 1) + it1] : 0.f;
+  const int role = adj0 ? 0 : 1;
+  edge_send<TX>(T, r, role, p, (unsigned)(it1 + 1));
+  publish_p<TX>(T, r, p);
+  publish_uw<TX>(T, r, u, w);
+  __syncthreads();
+  // Inputs of step it, fetched a step ahead by the adjoint threads: adjoint sources; strips of step it-1,
+  // the side arrays in bands with (or next to) columns L+1, L+2 / NX-L-1, NX-L.
+  {
+    const StripOff o = strip_offsets(g.nx, g.nz);
+    const int jx0 = tt0 * TX + 1 - L, lo = max(0, 1 - jx0), fn = nr ? max(0, min(n * TX, g.nx - jx0 + 1) - lo) : 0;
+    const int xa = tt0 * TX + 1 - 3, xb = (tt0 + n) * TX + 3;
+    for (int a = tid >> 5; a < 13; a += nthr >> 5) {
+      if (a < 6) {
+        const int to = 4 * ((a < 3 ? r.W : 0) + lo) + (a < 3 ? a : a - 2);
+        const int from = (a < 3 ? a * g.nx : o.T0 + (a - 3) * g.nx) + jx0 + lo - 1;
+        list_append(r, s_cnt + 1, fn, [&](int i) { return make_int2(to + 4 * i, from + i); });
+      } else if (a < 12) {
+        if (nr && (a < 9 ? (xa <= L + 2 && xb >= L + 1) : (xa <= NX - L && xb >= NX - L - 1)))
+          list_append(r, s_cnt + 1, g.nz, [&](int i) {
+            return make_int2(4 * (2 * r.W + (a - 6) * r.nqr) + 1 + i, o.S0 + (a - 6) * g.nz + i);
+          });
+      } else {
+        // entries without a receiver (the padding of a tile's entries) repeat receiver 0: never read
+        list_append(r, s_cnt + 1, s_cnt[0],
+                    [&](int i) { return make_int2(4 * (2 * r.W + 6 * r.nqr) + i, ~s_ig[i]); });
+      }
+    }
+  }
+  __syncthreads();
+  const int nlist = s_cnt[1];
+  auto prefetch = [&](int it) {
+    const size_t so = opaque(s);
+    const float* at = adj_t + (so * g.nt + (it - 1)) * g.ngmax;
+    const float* bs = strips + (so * g.snt + (it - 1 - g.sit0)) * g.SL;
+    float* box = res_smf() + 4 * box_at(r, it);
+    for (int i = tid; i < nlist; i += r.nA) {
+      const int2 q = res_list(r)[i];
+      cp4(box + q.x, q.y < 0 ? at + ~q.y : bs + q.y);
+    }
+  };
+  const bool rare = __any_sync(0xffffffffu, (T.f & (kLeft | kRight | kEnds | kStrip | kRec)) || isrc >= 0 || gu);
+  if (rare) T.f |= kRare;
+  if (T.f & kAdj) {
+    prefetch(it1);
+    cp_wait();
+  }
+  __syncthreads();
+  auto image = [&]() {  // the step before: image and illumination of the reconstruction
+#pragma unroll
+    for (int c = 0; c < TX; ++c) {
+      float d[4];
+      lds4(r.oD + (TX + 1) * T.slot + c, d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s1[c][j] = s1[c][j] + p[c][j] * d[j];
+        s2[c][j] = s2[c][j] + p[c][j] * p[c][j];
+      }
+    }
+  };
+  bool dead = false;
+
+  for (int it = it1; it >= it0; --it) {
+    // ---- velocity phase
+    if (!(T.f & kAdj) && it < it1) image();
+    if (T.f & kSide)
+      tile_w<TX, true>(T, r, tt0, p, w, c1, c2);
+    else
+      tile_w<TX, false>(T, r, tt0, p, w, c1, c2);
+    if (T.f & kAdj) {
+      // outside the update range of w both rows are never read
+#pragma unroll
+      for (int c = 0; c < TX; ++c) mov_if(T.f & kTopFs, w[c][0], w[c][1]);
+      if (it > it0) prefetch(it - 1);
+    } else {
+      const int at = strip_b(r, it) + opaque(T.ix0) - 1 - tt0 * TX;
+      SWIT_RES_ROW(r.jz, insert_row<TX>(T.f & kB1, at, 2, w, (J + 3) & 3))
+    }
+    if (T.f & kRare) {
+      edge_recv<TX>(T, r, role, role ? r.oGR : r.oG, gu, dead, p, (unsigned)(it + 1), c1, c2);
+      if (gu >> 4) {  // ghost columns jx = 1 and nx-1 of the reconstruction
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          if ((gu >> q) & 0x110u) {
+            const int slot = q < 2 ? T.e - kEdge * r.nq + 3 + q : T.e + kEdge * r.nq + 5;
+            float v[4];
+            lds4(slot, v);
+            side_insert<TX>(T, r, it, (gu >> q) & 16u ? 2 : 5, v);
+            res_sm[slot] = mk4(v);
+          }
+      }
+    }
+    __syncwarp();
+    if (T.f & kSide)
+      tile_u<TX, true>(T, r, tt0, p, u, c1, c2);
+    else
+      tile_u<TX, false>(T, r, tt0, p, u, c1, c2);
+    if (T.f & kRare) {
+      if (T.f & kEnds) zero_cols<TX>(T.ix0, u, 2, NX - 2);
+      if ((T.f & (kStrip | kAdj)) == kStrip) {
+#pragma unroll
+        for (int c = 0; c < TX; ++c) {
+          const int ix = T.ix0 + c;
+          if (ix == L + 1 || ix == NX - L - 1) side_insert<TX>(T, r, it, ix == L + 1 ? 2 : 5, u[c]);
+        }
+      }
+    }
+    publish_uw<TX>(T, r, u, w);
+    __syncthreads();
+    // ---- pressure phase
+    if (T.f & kAdj) {
+#pragma unroll
+      for (int c = 0; c < TX; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s2[c][j] = p[c][j];
+    } else if ((T.f & kRare) && isrc >= 0) {
+      add_at<TX, true>(p, isrc, g.dt * snext);
+      snext = s_fwd[(size_t)s * (g.nt + 1) + it - 1];
+    }
+    if (T.f & kSide)
+      tile_p<TX, true>(T, r, tt0, p, u, w, c1, c2);
+    else
+      tile_p<TX, false>(T, r, tt0, p, u, w, c1, c2);
+    if (T.f & kAdj) {
+      if ((T.f & kRare) && (T.f & kEnds)) zero_cols<TX>(T.ix0, p, 3, NX - 2);
+      if (rec.comp == 0) {
+        rec_add_line<TX, false>(R, p, box_adj(r, it), g.dt);
+        if ((T.f & kRare) && (T.f & kRec)) rec_add<TX, false>(R, p, s_code, res_smf() + 4 * box_adj(r, it), g.dt);
+      }
+#pragma unroll
+      for (int c = 0; c < TX; ++c) mov_if(T.f & kTop, p[c][0], -p[c][2]);
+    } else {
+      // re-insert in the reference's order: bottom, sides, top.  Every pressure the reference does not
+      // update is re-inserted, and no update that survives reads a velocity it does not update, apart
+      // from the re-inserted ones (w row nz-1, u columns 1 and nx-1): no update range is tested.
+      const int xl = opaque(T.ix0) - 1 - tt0 * TX;
+      const int at = strip_b(r, it) + xl;
+      SWIT_RES_ROW(r.jz, insert_row<TX>(T.f & kB0, at, 0, p, J); insert_row<TX>(T.f & kB1, at, 1, p, (J + 3) & 3))
+      if ((T.f & kRare) && (T.f & kStrip)) {
+#pragma unroll
+        for (int c = 0; c < TX; ++c) {
+          const int ix = T.ix0 + c;
+          // with nx >= 8 the four columns are distinct
+          const int a = ix == L + 1 ? 0 : (ix == L + 2 ? 1 : (ix == NX - L ? 3 : (ix == NX - L - 1 ? 4 : -1)));
+          if (a >= 0) side_insert<TX>(T, r, it, a, p[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < TX; c += 4) lds4x3_if(T.f & kTop, strip_t(r, it) + xl + c, p[c], p[c + 1], p[c + 2], p[c + 3]);
+    }
+    if (T.f & kRare)     edge_send<TX>(T, r, role, p, (unsigned)it);
+    publish_p<TX>(T, r, p);
+    if (T.f & kAdj) {
+#pragma unroll
+      for (int c = 0; c < TX; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s2[c][j] = s2[c][j] - p[c][j];
+          s1[c][j] = s1[c][j] + p[c][j] * p[c][j];
+        }
+      put_cols<TX>(T.f & kImg, r.oD + (TX + 1) * T.slot, s2);
+      // vz receivers: the adjoint source changes w after the pressure phase (vx: not on this path)
+      if (rec.comp == 2) {
+        rec_add_line<TX, true>(R, w, box_adj(r, it), g.dt);
+        if ((T.f & kRare) && (T.f & kRec)) rec_add<TX, true>(R, w, s_code, res_smf() + 4 * box_adj(r, it), g.dt);
+      }
+    }
+    if (T.f & kAdj) cp_wait();
+    __syncthreads();
+  }
+  const bool adj = T.f & kAdj, live = T.f & kLive;
+  if (!adj) image();
+  const int iz0 = row0<TX>(T, r, fs);
+  const int z0 = adj ? 1 : L + 1, z1 = adj ? NZ : L + g.nz, x0 = adj ? 1 : L + 1, x1 = adj ? NX : L + g.nx;
+  tile_store<TX>((adj ? PB : PE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, p);
+  tile_store<TX>((adj ? UB : UE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, u);
+  tile_store<TX>((adj ? WB : WE) + off, g.LD, T.ix0, iz0, live, z0, z1, x0, x1, w);
+  tile_store<TX>((adj ? DBK : DG) + off, g.LD, T.ix0, iz0, live, L + 1, L + g.nz, L + 1, L + g.nx, s1);
+  tile_store<TX>(DFW + off, g.LD, T.ix0, iz0, live && !adj, L + 1, L + g.nz, L + 1, L + g.nx, s2);
+}
+
 }  // namespace swit

@@ -15,14 +15,19 @@ namespace {
 
 using ResFwdFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, const float*, float*, float*, float*, float*,
                           float*, int, int, int);
+using ResBwdFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, const float*, const float*, float*, float*, float*,
+                          float*, float*, float*, float*, float*, float*, const float*, int, int, int);
+
 struct ResInst {
   int tx, maxt;
   ResFwdFn f;
+  ResBwdFn b;
 };
 inline const ResInst* res_instances(bool bwd, int& n) {
-  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512>}};
-  n = bwd ? 0 : (int)(sizeof(F) / sizeof(F[0]));
-  return F;
+  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512>, nullptr}};
+  static const ResInst B[] = {{4, 512, nullptr, k_bwd_res<4, 512>}, {4, 384, nullptr, k_bwd_res<4, 384>}};
+  n = bwd ? (int)(sizeof(B) / sizeof(B[0])) : (int)(sizeof(F) / sizeof(F[0]));
+  return bwd ? B : F;
 }
 
 // Split of a shot into bands of at most `tiles` column tiles, with the shared memory of a block.
@@ -130,7 +135,7 @@ inline void res_choose(const swit_engine* e, bool bwd, ResLoop& out) {
       lastC = r.C;
       if (r.nA + r.nR > I[i].maxt) break;
       if (r.smem > optin) continue;
-      const void* f = (const void*)I[i].f;
+      const void* f = bwd ? (const void*)I[i].b : (const void*)I[i].f;
       int occ = 0;
       if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, r.nA + r.nR, r.smem) != cudaSuccess) {
@@ -201,6 +206,22 @@ inline void res_forward(swit_engine* e, const ResLoop& l, bool store, int s0, in
     cudaLaunchKernelEx(&cfg, f, make_grid<float>(e), l.r, make_src(e), make_rec(e), (const float*)e->src,
                        (float*)e->p, (float*)e->u, (float*)e->w, (float*)e->seis_t,
                        store ? (float*)e->strips : (float*)nullptr, lo, hi, s);
+    if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
+  }
+}
+
+inline void res_backward(swit_engine* e, const ResLoop& l, int s0, int nb, cudaStream_t st, int hi, int lo,
+                         std::vector<cudaEvent_t>* ev = nullptr) {
+  if (lo > hi) return;
+  const ResBwdFn f = res_inst(true, l).b;
+  for (int s = s0; s < s0 + nb; s += l.shots) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = res_config(l, std::min(l.shots, s0 + nb - s), st, at);
+    if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
+    cudaLaunchKernelEx(&cfg, f, make_grid<float>(e), l.r, make_src(e), make_rec(e), (const float*)e->src,
+                       (const float*)e->adj_t, (float*)e->pb, (float*)e->ub, (float*)e->wb, (float*)e->pe,
+                       (float*)e->ue, (float*)e->we, (float*)e->dg, (float*)e->dfw, (float*)e->dbk,
+                       (const float*)e->strips, hi, lo, s);
     if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
   }
 }

@@ -63,6 +63,54 @@ def test_forward_matches_oracle(shape, tiles, monkeypatch):
         np.testing.assert_array_equal(snap[k], ref[k], err_msg=k)
 
 
+@pytest.mark.parametrize("shape,tiles", [(a, t) for a, t in SHAPES if a.get("comp") != "vx"])
+def test_reverse_matches_oracle(shape, tiles, monkeypatch):
+    s, pb = problem(**shape)
+    src, rho = s.source(), s.rho(s.vp_true)
+    ref = O.forward(pb, s.vp_true, rho, src, store=True)
+    adj = (np.random.default_rng(tiles).standard_normal(ref["seis"].shape) * 1e-3).astype(np.float32)
+    want = O.adjoint(pb, s.vp_true, rho, src, adj, ref)
+    split(monkeypatch, tiles)
+    with Engine(**s.engine_args(), receiver_component=shape.get("comp", "p")) as e:
+        assert e.query()["kernel"] == "resident"
+        e.set_model(s.vp_true, rho)
+        e.forward(src, save_boundary=True)
+        first = e.backward(adj)
+        again = e.backward(adj)
+        e.check()
+    for got in (first, again):
+        for a, k in zip(got, ("g", "fw", "bk")):
+            np.testing.assert_array_equal(a, want[k], err_msg=k)
+
+
+@pytest.mark.parametrize("every", [32, 50, 139, 140])
+def test_checkpointed_segments_match_oracle(every, monkeypatch):
+    """Segments of a checkpointed run start and end in the fields the loop before left in memory."""
+    s, pb = problem()
+    src, rho = s.source(), s.rho(s.vp_true)
+    ref = O.forward(pb, s.vp_true, rho, src, store=True)
+    adj = (ref["seis"] * 0.5).astype(np.float32)
+    want = O.adjoint(pb, s.vp_true, rho, src, adj, ref)
+    split(monkeypatch, 2)
+    with Engine(**s.engine_args(), checkpoint_every=every) as e:
+        assert e.query()["kernel"] == "resident"
+        e.set_model(s.vp_true, rho)
+        np.testing.assert_array_equal(e.forward(src, save_boundary=True), ref["seis"])
+        for a, k in zip(e.backward(adj), ("g", "fw", "bk")):
+            np.testing.assert_array_equal(a, want[k], err_msg=k)
+
+
+def test_routes():
+    """What the resident loops do not take stays on the step kernels."""
+    s, _ = problem()
+    for opts, kernel in ((dict(), "resident"), (dict(kernel="vec"), "vec"), (dict(shots_per_batch=1), "vec"),
+                         (dict(precision="fp64"), "vec"), (dict(path="plain"), "vec"), (dict(graph_branches=2), "vec"),
+                         (dict(block_x=8), "vec"), (dict(checkpoint_every=31), "vec"),
+                         (dict(receiver_component="vx"), "vec"), (dict(adjoint="exact"), "vec")):
+        with Engine(**s.engine_args(), **opts) as e:
+            assert e.query()["kernel"] == kernel, opts
+
+
 def test_halo_timeout_is_reported_and_the_context_stays_usable(monkeypatch):
     """With a poll limit of 0 every halo wait gives up at its first miss, records
     it in the engine's error word and goes on without waiting: the call with host
