@@ -1729,6 +1729,7 @@ struct swit_multi {
     cudaGraphExec_t g[3] = {nullptr, nullptr, nullptr};  // its forward (no strips, strips) and reverse loops
   };
   std::vector<Wave> waves;
+  std::vector<int> res_rows;  // table rows of the instances that run their resident loops
   size_t graph_nodes = size_t(1) << 20;  // kernel nodes per loop held in the waves' graphs, at most
   int branches = 3;
   cudaStream_t cap = nullptr, capx[2] = {nullptr, nullptr};
@@ -1758,6 +1759,12 @@ void multi_release(swit_multi* m) {
     delete e;
   }
 }
+
+// Instances whose two loops are resident run those, one launch per group of shots, spread over the branch
+// streams: the device schedules a cooperative launch whole, when its blocks fit beside those running, so
+// small problems share it.  6 uneven problems of up to 12 shots 701x251 (gradient): 177.9 ms in waves of the
+// step kernels, 144.1 ms with their resident loops.
+inline bool multi_resident(const swit_engine* e) { return e->resf && e->resb; }
 
 // Instance table, padded task lists, waves with their block tables and active
 // prefixes.  A wave's reverse-loop state stays under 0.7 L2 / branches (as the
@@ -1845,6 +1852,10 @@ int multi_build(swit_multi* m) {
   double used = 0.0;
   for (int r = 0; r < n; ++r) {
     const int ns = m->eng[m->order[r]]->ns;
+    if (multi_resident(m->eng[m->order[r]])) {  // no wave: its loops are launches of their own
+      m->res_rows.push_back(r);
+      continue;
+    }
     if (ns * state[r] <= 0.5 * budget) {
       if (used + ns * state[r] > budget && !shared.back().empty()) {
         shared.emplace_back();
@@ -1915,7 +1926,7 @@ int multi_build(swit_multi* m) {
     CK(cudaMalloc(&m->d_blocks[k], std::max<size_t>(B[k].size(), 1) * sizeof(uint2)));
     CK(cudaMemcpy(m->d_blocks[k], B[k].data(), B[k].size() * sizeof(uint2), cudaMemcpyHostToDevice));
   }
-  m->branches = std::max(1, std::min(m->branches, (int)m->waves.size()));
+  m->branches = std::max(1, std::min(m->branches, (int)(m->waves.size() + m->res_rows.size())));
   CK(cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking));
   for (int i = 0; i < 2; ++i) {
     CK(cudaStreamCreateWithFlags(&m->capx[i], cudaStreamNonBlocking));
@@ -1991,8 +2002,16 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
       return fail(SWIT_E_CUDA, "multi-instance graph: %s", cudaGetErrorString(rc));
     }
   }
+  // (work, row) of the switched-on instances with resident loops, most work first
+  std::vector<std::pair<double, int>> res;
+  for (int r : m->res_rows)
+    if (rows[r]) {
+      const swit_engine* e = m->eng[m->order[r]];
+      res.emplace_back((which < 2 ? e->resf : e->resb)->us * (e->nt - 1), r);
+    }
+  std::stable_sort(res.begin(), res.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
   // the waves on the branch streams, forked from and joined back to st
-  const int br = std::max(1, std::min(m->branches, (int)active.size()));
+  const int br = std::max(1, std::min(m->branches, (int)(active.size() + res.size())));
   auto branch = [&](int b) { return b ? m->capx[b - 1] : st; };
   CK(cudaEventRecord(m->ev_fork, st));
   for (int i = 0; i < br - 1; ++i) CK(cudaStreamWaitEvent(m->capx[i], m->ev_fork, 0));
@@ -2001,6 +2020,17 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
                    [&](int a, int b) { return m->waves[a].work > m->waves[b].work; });
   std::vector<double> load(br, 0.0);
   std::vector<std::vector<int>> direct(br);
+  for (const auto& q : res) {
+    const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[b] += q.first;
+    swit_engine* e = m->eng[m->order[q.second]];
+    if (which < 2)
+      res_forward(e, *e->resf, which == 1, 0, e->ns, branch(b), 2, e->nt);
+    else
+      res_backward(e, *e->resb, 0, e->ns, branch(b), e->nt, 2);
+  }
+  // waves count on from an even load: their work is in other units, and few calls hold both
+  if (!res.empty()) std::fill(load.begin(), load.end(), 0.0);
   for (int wi : by_work) {
     const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
     load[b] += m->waves[wi].work;
@@ -2080,8 +2110,6 @@ void auto_batches(swit_engine* e, int branches) {
 // which the resident reverse loop does not do.
 static int res_setup(swit_engine* e, const swit_desc* d) {
   if (d->kernel_variant || e->prec || e->path || d->shots_per_batch || d->graph_branches || d->block_x) return 0;
-  if (const char* v = std::getenv("SWIT_RESIDENT"))
-    if (std::atoi(v) == 0) return 0;
   if (e->ckpt_k && e->ckpt_k < 32) return 0;
   ResLoop f, b;
   res_choose(e, false, f);

@@ -8,6 +8,7 @@ struct ResLoop {
   bool ok = false;
   int tx = 0, maxt = 0;
   int shots = 0;  // per launch, at most
+  double us = 0.0;  // estimated microseconds per time step of all shots
   swit::ResPlan r{};
 };
 
@@ -154,6 +155,7 @@ inline void res_choose(const swit_engine* e, bool bwd, ResLoop& out) {
         out.tx = I[i].tx;
         out.maxt = I[i].maxt;
         out.shots = shots;
+        out.us = t;
         out.r = r;
       }
     }

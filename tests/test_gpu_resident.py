@@ -133,3 +133,44 @@ def test_halo_timeout_is_reported_and_the_context_stays_usable(monkeypatch):
         e.set_model(s.vp_true, rho)
         np.testing.assert_array_equal(e.forward(src, save_boundary=False), ref["seis"])
         e.check()
+
+
+@pytest.mark.parametrize("kernels,env", [(("auto", "vec", "auto"), {}), (("vec", "vec", "vec"), {}),
+                                         (("vec", "vec", "vec"), {"SWIT_MULTI_WAVE_BYTES": "1"}),
+                                         (("vec", "auto", "vec"), {"SWIT_MULTI_WAVE_BYTES": "5e5",
+                                                                   "SWIT_MULTI_GRAPH_NODES": "0"}),
+                                         (("vec", "vec", "vec"), {"SWIT_MULTI_WAVE_BYTES": "1",
+                                                                  "SWIT_MULTI_GRAPH_NODES": "300"})])
+def test_multi_engine_resident_and_wave_instances(kernels, env, monkeypatch):
+    """Instances with resident loops run beside instances in waves of the step
+    kernels (kernel="vec"), in every wave layout; every result equals the
+    instance's own engine's."""
+    import torch
+    from swit_gb300 import MultiEngine
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    shapes = [dict(nx=37, nz=28, npml=9, nt=120, ns=2), dict(nx=61, nz=41, npml=12, nt=150, ns=3),
+              dict(nx=30, nz=26, npml=8, nt=100, ns=1)]
+    probs, args = [problem(**k)[0] for k in shapes], []
+    for s, kernel in zip(probs, kernels):
+        args.append(dict(s.engine_args(), kernel=kernel))
+    srcs = [torch.from_numpy(s.source()).cuda() for s in probs]
+    obss = [torch.rand((s.ns, s.ng, s.nt), device="cuda", generator=torch.Generator("cuda").manual_seed(i)) * 1e-3
+            for i, s in enumerate(probs)]
+    want = []
+    for a, s, x, o in zip(args, probs, srcs, obss):
+        with Engine(**a) as e:
+            e.set_model(s.vp_true, s.rho(s.vp_true))
+            want.append((e.gradient_l2(x, o), e.misfit_l2(x, o)))
+    with MultiEngine(args) as m:
+        for e, s in zip(m.engines, probs):
+            e.set_model(s.vp_true, s.rho(s.vp_true))
+        got = m.gradient_l2(srcs, obss)
+        some = m.misfit_l2(srcs, obss, active=[True, False, True])
+        every = m.misfit_l2(srcs, obss)
+    for g, (w, v) in zip(got, want):
+        for k in ("grad", "illum_fw", "illum_bk"):
+            torch.testing.assert_close(g[k], w[k], rtol=0, atol=0)
+        assert g["misfit"] == w["misfit"]
+    assert every == [v for _, v in want]
+    assert some == [want[0][1], 0.0, want[2][1]]
