@@ -179,14 +179,6 @@ __device__ __forceinline__ void pkt_put(uint4* p, unsigned tag, float a, float b
       "r"(tag), "f"(a), "f"(b), "f"(c)
       : "memory");
 }
-__device__ __forceinline__ void pkt_get(const uint4* p, unsigned& tag, float& a, float& b, float& c) {
-  asm volatile(
-      "{\n\t.reg .b128 v;\n\t.reg .b64 lo, hi;\n\tld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {lo, hi}, v;\n\t"
-      "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
-      : "=r"(tag), "=f"(a), "=f"(b), "=f"(c)
-      : "l"(p)
-      : "memory");
-}
 // Three columns of one row tile.
 __device__ __forceinline__ void halo_put(uint4* p, int nq, unsigned tag, const float* a, const float* b,
                                          const float* c) {
@@ -195,16 +187,34 @@ __device__ __forceinline__ void halo_put(uint4* p, int nq, unsigned tag, const f
   pkt_put(p + 2 * nq, tag, b[2], b[3], c[0]);
   pkt_put(p + 3 * nq, tag, c[1], c[2], c[3]);
 }
-__device__ __forceinline__ void halo_get(const uint4* p, unsigned tag, const ResPlan& r, bool& dead, float* a,
-                                         float* b, float* c) {
-  const int nq = r.nq;
+// The four packets of a row tile as loaded.
+struct Halo {
+  unsigned t[4];
+  float a[4], b[4], c[4];
+};
+// Issues the loads; what they bring is looked at later (halo_wait).
+__device__ __forceinline__ void halo_issue(const uint4* p, int nq, Halo& h) {
+  auto get = [&](const uint4* q, unsigned& t, float& x, float& y, float& z) {
+    asm volatile(
+        "{\n\t.reg .b128 v;\n\t.reg .b64 lo, hi;\n\tld.relaxed.gpu.global.b128 v, [%4];\n\tmov.b128 {lo, hi}, v;\n\t"
+        "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+        : "=r"(t), "=f"(x), "=f"(y), "=f"(z)
+        : "l"(q)
+        : "memory");
+  };
+  get(p, h.t[0], h.a[0], h.a[1], h.a[2]);
+  get(p + nq, h.t[1], h.a[3], h.b[0], h.b[1]);
+  get(p + 2 * nq, h.t[2], h.b[2], h.b[3], h.c[0]);
+  get(p + 3 * nq, h.t[3], h.c[1], h.c[2], h.c[3]);
+}
+__device__ __forceinline__ bool halo_here(const Halo& h, unsigned tag) {
+  return h.t[0] == tag && h.t[1] == tag && h.t[2] == tag && h.t[3] == tag;
+}
+// Loads until the packets are those of the tag.
+__device__ __forceinline__ void halo_wait(const uint4* p, unsigned tag, const ResPlan& r, bool& dead, Halo& h) {
   for (unsigned n = 0;; ++n) {
-    unsigned t0, t1, t2, t3;
-    pkt_get(p, t0, a[0], a[1], a[2]);
-    pkt_get(p + nq, t1, a[3], b[0], b[1]);
-    pkt_get(p + 2 * nq, t2, b[2], b[3], c[0]);
-    pkt_get(p + 3 * nq, t3, c[1], c[2], c[3]);
-    if ((t0 == tag && t1 == tag && t2 == tag && t3 == tag) || dead) return;
+    halo_issue(p, r.nq, h);
+    if (halo_here(h, tag) || dead) return;
     if (n >= r.wait || ((n & 255u) == 255u && *(volatile int*)r.err != 0)) {
       atomicCAS(r.err, 0, kResErr);
       dead = true;
@@ -443,28 +453,41 @@ __device__ __forceinline__ void ghost_u(int slot, int coef, int fac, float c1, f
   res_sm[slot] = mk4(u);
 }
 
-// Receives the halo of p, puts its columns into the ghost slots of the edge
-// arrays and updates the ghost u.  gu: ghost columns whose u is updated (bits 0,
-// 1: left, 2: right); ghosts: the role's ghost tables.
+// Packets for this tile: from the left neighbour's right side, or the right one's left side.
 template <int TX>
+__device__ __forceinline__ const uint4* halo_from(const Tile<TX>& T, const ResPlan& r, int role, unsigned tag, bool left) {
+  return halo_at<TX>(T, r, role, tag) + (left ? kHaloSide - kHaloBlock : kHaloBlock) * r.nq;
+}
+// The reverse loop issues the loads for a tile at one edge before it updates w: by then the packets have
+// mostly arrived, and their latency (about 650 cycles) is covered (49 shots 481x141: 41.0 -> 39.1 us per
+// step).  The forward gets to that point too early for that: 14.2 against 15.5 us.
+template <int TX>
+__device__ __forceinline__ void edge_issue(const Tile<TX>& T, const ResPlan& r, int role, unsigned tag, Halo& h) {
+  if ((T.f & kRare) && (T.f & (kLeft | kRight))) halo_issue(halo_from<TX>(T, r, role, tag, T.f & kLeft), r.nq, h);
+}
+
+// Waits for the halo of p, puts its columns into the ghost slots of the edge
+// arrays and updates the ghost u.  gu: ghost columns whose u is updated (bits 0,
+// 1: left, 2: right); ghosts: the role's ghost tables; EARLY: h holds loads issued for the left edge, or for
+// the right one where that is the tile's only one.
+template <int TX, bool EARLY>
 __device__ __forceinline__ void edge_recv(const Tile<TX>& T, const ResPlan& r, int role, int ghosts, unsigned gu,
-                                          bool& dead, const float (&p)[TX][4], unsigned tag, float c1, float c2) {
+                                          bool& dead, const float (&p)[TX][4], unsigned tag, float c1, float c2,
+                                          Halo& h) {
   if (!(T.f & (kLeft | kRight))) return;
-  const uint4* o = halo_at<TX>(T, r, role, tag);
   const int nq = r.nq, g = ghosts + kEdge * opaque(T.k), e = opaque(T.e), el = e - kEdge * nq, er = e + kEdge * nq;
-  if (T.f & kLeft) {
-    float a[4], b[4], c[4];  // columns ix0-3, ix0-2, ix0-1
-    halo_get(o + (kHaloSide - kHaloBlock) * nq, tag, r, dead, a, b, c);
-    res_sm[el + 2] = mk4(c);
-    if (gu & 1u) ghost_u(el + 3, g, g + 3, c1, c2, a, b, c, p[0]);
-    if (gu & 2u) ghost_u(el + 4, g + 1, g + 4, c1, c2, b, c, p[0], p[1]);
+  if (T.f & kLeft) {  // columns ix0-3, ix0-2, ix0-1
+    if (!EARLY || !halo_here(h, tag)) halo_wait(halo_from<TX>(T, r, role, tag, true), tag, r, dead, h);
+    res_sm[el + 2] = mk4(h.c);
+    if (gu & 1u) ghost_u(el + 3, g, g + 3, c1, c2, h.a, h.b, h.c, p[0]);
+    if (gu & 2u) ghost_u(el + 4, g + 1, g + 4, c1, c2, h.b, h.c, p[0], p[1]);
   }
-  if (T.f & kRight) {
-    float a[4], b[4], c[4];  // columns ix0+TX .. ix0+TX+2
-    halo_get(o + kHaloBlock * nq, tag, r, dead, a, b, c);
-    res_sm[er] = mk4(a);
-    res_sm[er + 1] = mk4(b);
-    if (gu & 4u) ghost_u(er + 5, g + 2, g + 5, c1, c2, p[TX - 1], a, b, c);
+  if (T.f & kRight) {  // columns ix0+TX .. ix0+TX+2
+    if (!EARLY || (T.f & kLeft) || !halo_here(h, tag))
+      halo_wait(halo_from<TX>(T, r, role, tag, false), tag, r, dead, h);
+    res_sm[er] = mk4(h.a);
+    res_sm[er + 1] = mk4(h.b);
+    if (gu & 4u) ghost_u(er + 5, g + 2, g + 5, c1, c2, p[TX - 1], h.a, h.b, h.c);
   }
 }
 
@@ -883,7 +906,10 @@ __global__ void __launch_bounds__(MAXT, 1)
       tile_w<TX, false>(T, r, tt0, p, w, c1, c2);
 #pragma unroll
     for (int c = 0; c < TX; ++c) mov_if(T.f & kTopFs, w[c][0], w[c][1]);
-    if (T.f & kRare) edge_recv<TX>(T, r, 0, r.oG, gu, dead, p, (unsigned)it, c1, c2);
+    if (T.f & kRare) {
+      Halo h;
+      edge_recv<TX, false>(T, r, 0, r.oG, gu, dead, p, (unsigned)it, c1, c2, h);
+    }
     __syncwarp();
     if (T.f & kSide)
       tile_u<TX, true>(T, r, tt0, p, u, c1, c2);
@@ -1095,6 +1121,8 @@ __global__ void __launch_bounds__(MAXT, 1)
   for (int it = it1; it >= it0; --it) {
     // ---- velocity phase
     if (!(T.f & kAdj) && it < it1) image();
+    Halo h;
+    edge_issue<TX>(T, r, role, (unsigned)(it + 1), h);
     if (T.f & kSide)
       tile_w<TX, true>(T, r, tt0, p, w, c1, c2);
     else
@@ -1109,7 +1137,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       SWIT_RES_ROW(r.jz, insert_row<TX>(T.f & kB1, at, 2, w, (J + 3) & 3))
     }
     if (T.f & kRare) {
-      edge_recv<TX>(T, r, role, role ? r.oGR : r.oG, gu, dead, p, (unsigned)(it + 1), c1, c2);
+      edge_recv<TX, true>(T, r, role, role ? r.oGR : r.oG, gu, dead, p, (unsigned)(it + 1), c1, c2, h);
       if (gu >> 4) {  // ghost columns jx = 1 and nx-1 of the reconstruction
 #pragma unroll
         for (int q = 0; q < 3; ++q)
