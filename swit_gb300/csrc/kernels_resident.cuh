@@ -71,6 +71,7 @@ struct ResPlan {
   int W;         // columns of the widest band
   int ns;        // slots: (tiles of the widest band + 2) nq
   int jz;        // row nz within its tile
+  float negz;    // -0 (see f2)
   unsigned wait; // polls before a halo wait gives up
   uint4* halo;   // packets: [block][role][side][parity][packet][row tile]
   int* err;
@@ -290,6 +291,32 @@ __device__ __forceinline__ float2 col_factor(const Tile<TX>& T, const ResPlan& r
   return reinterpret_cast<const float2*>(res_sm + r.oX)[T.ix0 - 1 - tt0 * TX + c];
 }
 
+// Two FP32 operations per instruction (f32x2), each rounded as the scalar one.  Products are fma(x, y, -0)
+// with a -0 the compiler cannot see, for ptxas contracts a packed product and a following packed sum even
+// under --fmad=false; differences are fma(b, -1, a).  Rows j, j+1 of a column pair up without moves in the
+// x-differences and the products, so u is packed in every loop (forward step of 49 shots 481x141 with
+// strips 16.6 -> 16.2 us, of one shot 101x51 2.09 -> 1.98 us).  The operands of z-differences straddle
+// pairs: w's stay scalar and only its products and sums are packed, in the reverse loop (38.0 -> 37.6 us,
+// one shot 2.66 -> 2.42 us; in the forward loop it costs, 1.98 -> 2.08 us).  p, mostly z- and x-differences
+// of separate arrays, is scalar: its moves cost more than the sums save (14.8 against 14.3 us).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // The updates of a tile, the same code for every role: f := factor f - coef D (the reconstruction, which
 // adds without damping, has factor 1 and negated coefficients: the same values).
 //
@@ -332,7 +359,7 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
 }
 
 // w from p.
-template <int TX, bool SIDE>
+template <int TX, bool SIDE, bool PACK>
 __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int tt0, const float (&p)[TX][4],
                                        float (&w)[TX][4], float c1, float c2) {
   const int lane = threadIdx.x & 31;
@@ -341,6 +368,7 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
   zrow_get<TX>(r, -1, 0, e0);
   zrow_get<TX>(r, 1, 1, e5);
   zrow_get<TX>(r, 1, 2, e6);
+  const f2 Z = pk(r.negz, r.negz), C1 = pk(c1, c1), C2 = pk(c2, c2);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
     float a[4], fx = 1.f;
@@ -355,10 +383,26 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
     z[6] = lane == 31 ? e6[c] : z[6];
 #pragma unroll
     for (int j = 0; j < 4; ++j) z[1 + j] = p[c][j];
+    if constexpr (!PACK) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float D = c1 * (z[j + 2] - z[j + 1]) + c2 * (z[j + 3] - z[j]);
-      sub_if(bit_at(T.f, kW + j), w[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * w[c][j], a[j] * D);
+      for (int j = 0; j < 4; ++j) {
+        const float D = c1 * (z[j + 2] - z[j + 1]) + c2 * (z[j + 3] - z[j]);
+        sub_if(bit_at(T.f, kW + j), w[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * w[c][j], a[j] * D);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        const f2 d1 = pk(z[j + 2] - z[j + 1], z[j + 3] - z[j + 2]), d2 = pk(z[j + 3] - z[j], z[j + 4] - z[j + 1]);
+        const f2 D = add2(fma2(C1, d1, Z), fma2(C2, d2, Z));
+        const f2 S = fma2(pk(a[j], a[j + 1]), D, Z);
+        const f2 F = SIDE ? pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1])) : pk(fz[j], fz[j + 1]);
+        const f2 Q = fma2(F, pk(w[c][j], w[c][j + 1]), Z);
+        float s0, s1, q0, q1;
+        upk(S, s0, s1);
+        upk(Q, q0, q1);
+        sub_if(bit_at(T.f, kW + j), w[c][j], q0, s0);
+        sub_if(bit_at(T.f, kW + j + 1), w[c][j + 1], q1, s1);
+      }
     }
   }
 }
@@ -372,18 +416,24 @@ __device__ __forceinline__ void tile_u(const Tile<TX>& T, const ResPlan& r, int 
   lds4(T.e - kEdge * r.nq + 2, pm1);
   lds4(T.e + kEdge * r.nq, pp1);
   lds4(T.e + kEdge * r.nq + 1, pp2);
+  const f2 Z = pk(r.negz, r.negz), M = pk(-1.f, -1.f), C1 = pk(c1, c1), C2 = pk(c2, c2);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
     float a[4], fx = 1.f;
     lds4(r.oC + (2 * TX + 1) * threadIdx.x + TX + c, a);
     if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).y;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float l1 = c >= 1 ? p[c >= 1 ? c - 1 : 0][j] : pm1[j];
-      const float r1 = c + 1 < TX ? p[c + 1 < TX ? c + 1 : 0][j] : pp1[j];
-      const float r2 = c + 2 < TX ? p[c + 2 < TX ? c + 2 : 0][j] : (c + 1 < TX ? pp1[j] : pp2[j]);
-      const float D = c1 * (r1 - p[c][j]) + c2 * (r2 - l1);
-      u[c][j] = (SIDE ? fminf(fx, fz[j]) : fz[j]) * u[c][j] - a[j] * D;
+    for (int j = 0; j < 4; j += 2) {
+      auto P = [&](int k) {
+        const float* q = k < 0 ? pm1 : (k < TX ? p[k < 0 || k >= TX ? 0 : k] : (k == TX ? pp1 : pp2));
+        return pk(q[j], q[j + 1]);
+      };
+      const f2 d1 = fma2(P(c), M, P(c + 1)), d2 = fma2(P(c - 1), M, P(c + 2));
+      const f2 D = add2(fma2(C1, d1, Z), fma2(C2, d2, Z));
+      const f2 S = fma2(pk(a[j], a[j + 1]), D, Z);
+      const f2 F = SIDE ? pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1])) : pk(fz[j], fz[j + 1]);
+      const f2 U = fma2(S, M, fma2(F, pk(u[c][j], u[c][j + 1]), Z));
+      upk(U, u[c][j], u[c][j + 1]);
     }
   }
 }
@@ -901,9 +951,9 @@ __global__ void __launch_bounds__(MAXT, 1)
     __syncthreads();
     // ---- velocity phase
     if (T.f & kSide)
-      tile_w<TX, true>(T, r, tt0, p, w, c1, c2);
+      tile_w<TX, true, false>(T, r, tt0, p, w, c1, c2);
     else
-      tile_w<TX, false>(T, r, tt0, p, w, c1, c2);
+      tile_w<TX, false, false>(T, r, tt0, p, w, c1, c2);
 #pragma unroll
     for (int c = 0; c < TX; ++c) mov_if(T.f & kTopFs, w[c][0], w[c][1]);
     if (T.f & kRare) {
@@ -1124,9 +1174,9 @@ __global__ void __launch_bounds__(MAXT, 1)
     Halo h;
     edge_issue<TX>(T, r, role, (unsigned)(it + 1), h);
     if (T.f & kSide)
-      tile_w<TX, true>(T, r, tt0, p, w, c1, c2);
+      tile_w<TX, true, true>(T, r, tt0, p, w, c1, c2);
     else
-      tile_w<TX, false>(T, r, tt0, p, w, c1, c2);
+      tile_w<TX, false, true>(T, r, tt0, p, w, c1, c2);
     if (T.f & kAdj) {
       // outside the update range of w both rows are never read
 #pragma unroll

@@ -34,6 +34,7 @@ inline const ResInst* res_instances(bool bwd, int& n) {
 // Split of a shot into bands of at most `tiles` column tiles, with the shared memory of a block.
 inline ResPlan res_plan(const swit_engine* e, bool bwd, int tx, int tiles) {
   ResPlan r{};
+  r.negz = -0.0f;
   r.nt_tiles = (e->NX + tx - 1) / tx;
   r.C = (r.nt_tiles + tiles - 1) / tiles;
   const int widest = (r.nt_tiles + r.C - 1) / r.C;
