@@ -24,7 +24,7 @@
 #include "kernels_band.cuh"
 #include "kernels_multi.cuh"
 #include "kernels_exact.cuh"
-#include "kernels_resident.cuh"
+#include "kernels_resident_exact.cuh"
 
 using namespace swit;
 
@@ -141,7 +141,7 @@ struct swit_engine {
   std::vector<cudaGraphExec_t> gxb;
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
   // resident time loops (kernels_resident.cuh), where the split fits the device; else the variant's kernels
-  ResLoop *resf = nullptr, *resb = nullptr;
+  ResLoop *resf = nullptr, *resb = nullptr, *resx = nullptr;  // forward, reverse, exact adjoint's reverse
   uint4* d_halo = nullptr;
 };
 
@@ -241,7 +241,8 @@ namespace {
 void res_free(swit_engine* e) {
   delete e->resf;
   delete e->resb;
-  e->resf = e->resb = nullptr;
+  delete e->resx;
+  e->resf = e->resb = e->resx = nullptr;
 }
 
 // Launch shape of the stencil kernels for a batch of nb shots.
@@ -555,7 +556,11 @@ XAdj<R> make_xadj(swit_engine* e) {
 }
 
 template <class R>
-void launch_exact_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int it_hi, int it_lo) {
+void launch_exact_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int it_hi, int it_lo, bool res = false) {
+  if (res) {
+    res_xadj(e, *e->resx, make_xadj<float>(e), shot0, nb, st, it_hi, it_lo);
+    return;
+  }
   Grid<R> g = make_grid<R>(e);
   const XAdj<R> x = make_xadj<R>(e);
   const dim3 block = vec_block(e), g0 = vec_grid(e, 0, nb), g1 = vec_grid(e, 1, nb);
@@ -574,9 +579,9 @@ void launch_exact_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, int 
 // it, re-run its forward steps storing D into the k-step buffer, then run the
 // same steps in reverse.  Leaves sit0 = 1.
 template <class R>
-void exact_reverse(swit_engine* e, int s0, int nb, cudaStream_t st) {
+void exact_reverse(swit_engine* e, int s0, int nb, cudaStream_t st, bool res = false) {
   if (!e->ckpt_k) {
-    launch_exact_steps<R>(e, s0, nb, st, e->nt, 2);
+    launch_exact_steps<R>(e, s0, nb, st, e->nt, 2, res);
     return;
   }
   const int k = e->ckpt_k;
@@ -592,8 +597,8 @@ void exact_reverse(swit_engine* e, int s0, int nb, cudaStream_t st) {
       cudaMemsetAsync((char*)e->w + (size_t)s0 * fsz, 0, (size_t)nb * fsz, st);
     }
     e->sit0 = m * k + 1;
-    launch_forward_steps<R>(e, true, s0, nb, st, lo, hi);
-    launch_exact_steps<R>(e, s0, nb, st, hi, lo);
+    launch_forward_steps<R>(e, true, s0, nb, st, lo, hi, res);
+    launch_exact_steps<R>(e, s0, nb, st, hi, lo, res);
   }
   e->sit0 = 1;
 }
@@ -717,7 +722,8 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  if (e->resf && !(store && e->exact && !e->ckpt_k)) {  // the storing exact forward keeps D of every step
+  // the exact adjoint's forward keeps D of every step in its reverse loop's layout
+  if (e->resf && !(store && e->exact && !e->ckpt_k && !e->resx)) {
     if (store && e->ckpt_k)
       forward_checkpointed<R>(e, 0, e->ns, st, true);
     else
@@ -869,6 +875,11 @@ template <class R>
 int run_exact_loop(swit_engine* e, cudaStream_t st) {
   if (e->path == 1) {
     for (int s = 0; s < e->ns; ++s) exact_reverse<R>(e, s, 1, st);
+    CK(cudaGetLastError());
+    return 0;
+  }
+  if (e->resx) {
+    exact_reverse<R>(e, 0, e->ns, st, true);
     CK(cudaGetLastError());
     return 0;
   }
@@ -2111,11 +2122,12 @@ void auto_batches(swit_engine* e, int branches) {
 static int res_setup(swit_engine* e, const swit_desc* d) {
   if (d->kernel_variant || e->prec || e->path || d->shots_per_batch || d->graph_branches || d->block_x) return 0;
   if (e->ckpt_k && e->ckpt_k < 32) return 0;
-  ResLoop f, b;
-  res_choose(e, false, f);
-  if (!e->exact && e->rcomp != 1) res_choose(e, true, b);
+  ResLoop f, b, x;
+  res_choose(e, kResLoopFwd, f);
+  if (!e->exact && e->rcomp != 1) res_choose(e, kResLoopBwd, b);
+  if (e->exact && !e->rcomp && f.ok) res_choose(e, kResLoopXadj, x);
   if (e->ckpt_k && !e->exact && !(f.ok && b.ok)) return 0;
-  const size_t n = std::max(res_halo_packets(f), res_halo_packets(b));
+  const size_t n = std::max(std::max(res_halo_packets(f), res_halo_packets(b)), res_halo_packets(x));
   if (!n) return 0;
   if (int rc = dalloc(e, &e->d_halo, n)) return rc;
   unsigned wait = kResWaitLimit;
@@ -2123,11 +2135,12 @@ static int res_setup(swit_engine* e, const swit_desc* d) {
     const long long w = std::atoll(v);
     if (w >= 0 && w < (long long)kResWaitLimit) wait = (unsigned)w;
   }
-  f.r.halo = b.r.halo = e->d_halo;
-  f.r.err = b.r.err = e->d_err;
-  f.r.wait = b.r.wait = wait;
+  f.r.halo = b.r.halo = x.r.halo = e->d_halo;
+  f.r.err = b.r.err = x.r.err = e->d_err;
+  f.r.wait = b.r.wait = x.r.wait = wait;
   if (f.ok) e->resf = new ResLoop(f);
   if (b.ok) e->resb = new ResLoop(b);
+  if (x.ok) e->resx = new ResLoop(x);
   return 0;
 }
 
@@ -2187,7 +2200,8 @@ int swit_create(const swit_desc* d, swit_engine** out) {
     return fail(SWIT_E_ARG, "vx / vz receivers run on the walk or vec kernels (kernel_variant 0, 2 or 3)");
   }
   e->rcomp = d->receiver_component;
-  if (e->exact) e->SL = e->NX * e->LD;  // the strip buffer holds D of each step
+  // the strip buffer holds D of each step, in the fields' layout or by 4 x 4 tiles from row fs-1 (resident loops)
+  if (e->exact) e->SL = std::max(e->NX * e->LD, round_up(e->NX, 4) * round_up(e->NZ - e->fs + 2, 4));
   if (e->variant == 2) {
     e->bx = d->block_x > 0 ? d->block_x : 8;  // columns per tile
     if (e->bx < 2 || e->bx > 256) {
@@ -2457,9 +2471,9 @@ int swit_create(const swit_desc* d, swit_engine** out) {
   e->launches_bwd = e->variant == 4 ? per : per * (e->nt - 1) * per_step * (e->ckpt_k ? 2 : 1);
   const int segs = std::max(1, e->ckpt_m);
   const int resf = e->resf ? segs * ((ns + e->resf->shots - 1) / e->resf->shots) : 0;
-  if (e->resf && !(e->exact && !e->ckpt_k)) e->launches_fwd = resf;
-  if (e->resb)
-    e->launches_bwd = segs * ((ns + e->resb->shots - 1) / e->resb->shots) + (e->ckpt_k ? resf : 0);
+  if (e->resf && !(e->exact && !e->ckpt_k && !e->resx)) e->launches_fwd = resf;
+  if (const ResLoop* l = e->resb ? e->resb : e->resx)
+    e->launches_bwd = segs * ((ns + l->shots - 1) / l->shots) + (e->ckpt_k ? resf : 0);
   *out = e;
   return 0;
 }
@@ -2620,7 +2634,7 @@ int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_b
   if (block_x) *block_x = e->bx;
   if (kernels_per_forward) *kernels_per_forward = e->launches_fwd;
   if (kernels_per_backward) *kernels_per_backward = e->launches_bwd;
-  if (kernel_variant) *kernel_variant = e->resf && e->resb ? 7 : e->variant;
+  if (kernel_variant) *kernel_variant = e->resf && (e->resb || e->resx) ? 7 : e->variant;
   return 0;
 }
 

@@ -160,6 +160,11 @@ __device__ __forceinline__ void lds4x1_if(bool on, int i, int k, float& a, float
       : "r"((unsigned)on), "r"(res_addr(i) + 4u * k)
       : "memory");
 }
+__device__ __forceinline__ void stg4_if(unsigned on, float4* p, const float* v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.global.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"(on),
+               "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+               : "memory");
+}
 // v = a - b, v = v + a.
 __device__ __forceinline__ void sub_if(unsigned on, float& v, float a, float b) {
   asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t@q sub.rn.f32 %0, %1, %2;\n\t}" : "+f"(v) : "f"(a), "f"(b), "r"(on));
@@ -321,9 +326,11 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 // adds without damping, has factor 1 and negated coefficients: the same values).
 //
 // p from u (x-neighbours in the edge arrays) and w.
-template <int TX, bool SIDE>
+// SAVE: D of the tile to save[column of the tile * (column tiles of the shot) nq].
+template <int TX, bool SIDE, bool SAVE = false>
 __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int tt0, float (&p)[TX][4],
-                                       const float (&u)[TX][4], const float (&w)[TX][4], float c1, float c2) {
+                                       const float (&u)[TX][4], const float (&w)[TX][4], float c1, float c2,
+                                       float4* save = nullptr) {
   const int lane = threadIdx.x & 31;
   float um2[4], um1[4], up1[4], fz[4], e1[TX], e2[TX], e6[TX];
   lds4(T.rf, fz);
@@ -347,6 +354,7 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
     z[6] = lane == 31 ? e6[c] : z[6];
 #pragma unroll
     for (int j = 0; j < 4; ++j) z[2 + j] = w[c][j];
+    float d[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float l1 = c >= 1 ? u[c >= 1 ? c - 1 : 0][j] : um1[j];
@@ -354,7 +362,9 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
       const float r1 = c + 1 < TX ? u[c + 1 < TX ? c + 1 : 0][j] : up1[j];
       const float D = c1 * (u[c][j] - l1 + z[j + 2] - z[j + 1]) + c2 * (r1 - l2 + z[j + 3] - z[j]);
       sub_if(bit_at(T.f, kP + j), p[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * p[c][j], a[j] * D);
+      d[j] = D;
     }
+    if constexpr (SAVE) stg4_if(T.f & kLive, save + c * r.nt_tiles * r.nq, d);
   }
 }
 
@@ -811,12 +821,12 @@ __device__ __forceinline__ void list_append(const ResPlan& r, int* cnt, int n, F
 // stencil's): 512 threads of 128 registers hold as many points as the register file, so a launch takes as
 // many shots as the device holds.  Measured against the vec kernels: 49 shots 481x141, nt 2000, misfit only
 // 56.6 -> 29.3 ms; one shot 101x51, nt 600: 3.05 -> 1.20 ms.
-template <int TX, int MAXT>
+template <int TX, int MAXT, bool SAVE>
 __global__ void __launch_bounds__(MAXT, 1)
     k_fwd_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,
               const __grid_constant__ Sources src, const __grid_constant__ Receivers rec, const float* __restrict__ s_fwd,
               float* __restrict__ P, float* __restrict__ U, float* __restrict__ W_, float* __restrict__ seis_t,
-              float* __restrict__ strips, int it0, int it1, int shot0) {
+              float* __restrict__ strips, float4* __restrict__ dsave, int it0, int it1, int shot0) {
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
   const int b = blockIdx.x % r.C, s = shot0 + blockIdx.x / r.C;
   const int per = r.nt_tiles / r.C, rem = r.nt_tiles % r.C;
@@ -932,10 +942,13 @@ __global__ void __launch_bounds__(MAXT, 1)
 
   for (int it = it0; it <= it1; ++it) {
     // ---- pressure phase
+    float4* save = nullptr;
+    if constexpr (SAVE)
+      save = dsave + ((size_t)opaque(s) * g.snt + (it - g.sit0)) * (g.SL / 4) + (T.ix0 - 1) / TX * nq + T.k;
     if (T.f & kSide)
-      tile_p<TX, true>(T, r, tt0, p, u, w, c1, c2);
+      tile_p<TX, true, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
     else
-      tile_p<TX, false>(T, r, tt0, p, u, w, c1, c2);
+      tile_p<TX, false, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
     if (T.f & kRare) {
       if (T.f & kEnds) zero_cols<TX>(T.ix0, p, 3, NX - 2);
       if (isrc >= 0) {

@@ -15,24 +15,33 @@ struct ResLoop {
 namespace {
 
 using ResFwdFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, const float*, float*, float*, float*, float*,
-                          float*, int, int, int);
+                          float*, float4*, int, int, int);
 using ResBwdFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, const float*, const float*, float*, float*, float*,
                           float*, float*, float*, float*, float*, float*, const float*, int, int, int);
 
+using ResXadjFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, XAdj<float>, int, int, int);
+
+enum ResKind { kResLoopFwd, kResLoopBwd, kResLoopXadj };
+
 struct ResInst {
   int tx, maxt;
-  ResFwdFn f;
+  ResFwdFn f, fd;  // forward; the one that keeps D of every step for the exact adjoint
   ResBwdFn b;
+  ResXadjFn x;
+  const void* any() const { return f ? (const void*)f : (b ? (const void*)b : (const void*)x); }
 };
-inline const ResInst* res_instances(bool bwd, int& n) {
-  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512>, nullptr}};
-  static const ResInst B[] = {{4, 512, nullptr, k_bwd_res<4, 512>}, {4, 384, nullptr, k_bwd_res<4, 384>}};
-  n = bwd ? (int)(sizeof(B) / sizeof(B[0])) : (int)(sizeof(F) / sizeof(F[0]));
-  return bwd ? B : F;
+inline const ResInst* res_instances(ResKind kind, int& n) {
+  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512, false>, k_fwd_res<4, 512, true>, nullptr, nullptr}};
+  static const ResInst B[] = {{4, 512, nullptr, nullptr, k_bwd_res<4, 512>, nullptr},
+                              {4, 384, nullptr, nullptr, k_bwd_res<4, 384>, nullptr}};
+  static const ResInst X[] = {{4, 384, nullptr, nullptr, nullptr, k_xadj_res<4, 384>}};
+  n = kind == kResLoopBwd ? 2 : 1;
+  return kind == kResLoopFwd ? F : (kind == kResLoopBwd ? B : X);
 }
 
 // Split of a shot into bands of at most `tiles` column tiles, with the shared memory of a block.
-inline ResPlan res_plan(const swit_engine* e, bool bwd, int tx, int tiles) {
+inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
+  const bool bwd = kind == kResLoopBwd;
   ResPlan r{};
   r.negz = -0.0f;
   r.nt_tiles = (e->NX + tx - 1) / tx;
@@ -95,6 +104,12 @@ inline ResPlan res_plan(const swit_engine* e, bool bwd, int tx, int tiles) {
     r.oBox = take(2 * r.box);
     r.oEnt = take(1 + r.ent_cap / 2);  // counters, receivers, codes
     r.oList = take((6 * r.W + 6 * e->nz + r.ent_cap + 1) / 2);
+  } else if (kind == kResLoopXadj) {
+    r.oGR = take(kRow * r.nq);  // lu of the ghost columns
+    r.oD = take(tx * r.nA);
+    r.box = r.ent_cap / 4;
+    r.oBox = take(2 * r.box);
+    r.oEnt = take(1 + r.ent_cap / 2);
   } else {
     r.oStage = take(6 * r.W);
     r.oS = take(6 * r.nq);
@@ -109,37 +124,40 @@ inline ResPlan res_plan(const swit_engine* e, bool bwd, int tx, int tiles) {
 // measured steps (GB300, 32 to 512 threads per block): a fixed part, the dependent chain of a step
 // (updates, barriers, halo), and a part by the warps that share the SM.  A band of a single column tile
 // exchanges both its edges in the same threads; a shot in one band exchanges nothing.
-inline double res_step_us(const ResPlan& r, bool bwd, int maxt, int bpsm, int tiles) {
+inline double res_step_us(const ResPlan& r, ResKind kind, int maxt, int bpsm, int tiles) {
   const double warps = bpsm * ((r.nA + r.nR) / 32);
-  const double t = !bwd ? 1.55 + 0.09 * warps : 2.1 + (maxt > 384 ? 0.15 : 0.085) * warps;
+  const double t = kind == kResLoopXadj  ? 2.0 + 0.12 * warps
+                   : kind == kResLoopFwd ? 1.55 + 0.09 * warps
+                                         : 2.1 + (maxt > 384 ? 0.15 : 0.085) * warps;
   return t + (r.C > 1 ? (tiles == 1 ? 0.45 : 0.0) : -0.3);
 }
 
 // The fastest split by estimate among those whose blocks are co-resident.
-inline void res_choose(const swit_engine* e, bool bwd, ResLoop& out) {
+inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
   int dev = 0, sms = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return;
   int want = 0;  // column tiles per band instead of the estimate's choice, e.g. to test a split
-  if (const char* v = std::getenv(bwd ? "SWIT_RES_BWD_TILES" : "SWIT_RES_FWD_TILES")) want = std::atoi(v);
+  if (const char* v = std::getenv(kind != kResLoopFwd ? "SWIT_RES_BWD_TILES" : "SWIT_RES_FWD_TILES")) want = std::atoi(v);
   int ninst = 0;
-  const ResInst* I = res_instances(bwd, ninst);
+  const ResInst* I = res_instances(kind, ninst);
   double best = 0.0;
   for (int i = 0; i < ninst; ++i) {
     const int all = (e->NX + I[i].tx - 1) / I[i].tx;
     int lastC = -1;
     for (int tiles = 1; tiles <= all; ++tiles) {
       if (want && tiles != want) continue;
-      ResPlan r = res_plan(e, bwd, I[i].tx, tiles);
+      ResPlan r = res_plan(e, kind, I[i].tx, tiles);
       if (r.C == lastC) continue;
       lastC = r.C;
       if (r.nA + r.nR > I[i].maxt) break;
       if (r.smem > optin) continue;
-      const void* f = bwd ? (const void*)I[i].b : (const void*)I[i].f;
+      const void* f = e->exact && kind == kResLoopFwd ? (const void*)I[i].fd : I[i].any();
       int occ = 0;
-      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+      if (cudaFuncSetAttribute(I[i].any(), cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+          cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, r.nA + r.nR, r.smem) != cudaSuccess) {
         cudaGetLastError();
         continue;
@@ -149,7 +167,7 @@ inline void res_choose(const swit_engine* e, bool bwd, ResLoop& out) {
       const int waves = (e->ns + fit - 1) / fit;
       const int shots = (e->ns + waves - 1) / waves;
       const int bpsm = (shots * r.C + sms - 1) / sms;
-      const double t = waves * res_step_us(r, bwd, I[i].maxt, bpsm, (r.nt_tiles + r.C - 1) / r.C);
+      const double t = waves * res_step_us(r, kind, I[i].maxt, bpsm, (r.nt_tiles + r.C - 1) / r.C);
       if (!out.ok || t < best) {
         best = t;
         out.ok = true;
@@ -167,9 +185,9 @@ inline size_t res_halo_packets(const ResLoop& l) {
   return l.ok ? (size_t)l.shots * l.r.C * 2 * 2 * 2 * 4 * l.r.nq : 0;
 }
 
-inline const ResInst& res_inst(bool bwd, const ResLoop& l) {
+inline const ResInst& res_inst(ResKind kind, const ResLoop& l) {
   int n = 0;
-  const ResInst* I = res_instances(bwd, n);
+  const ResInst* I = res_instances(kind, n);
   for (int i = 0; i < n; ++i)
     if (I[i].tx == l.tx && I[i].maxt == l.maxt) return I[i];
   return I[0];
@@ -201,14 +219,16 @@ inline cudaEvent_t res_event() {
 inline void res_forward(swit_engine* e, const ResLoop& l, bool store, int s0, int nb, cudaStream_t st, int lo, int hi,
                         std::vector<cudaEvent_t>* ev = nullptr) {
   if (lo > hi) return;
-  const ResFwdFn f = res_inst(false, l).f;
+  const bool save = store && e->exact;  // the strip buffer holds D
+  const ResFwdFn f = save ? res_inst(kResLoopFwd, l).fd : res_inst(kResLoopFwd, l).f;
   for (int s = s0; s < s0 + nb; s += l.shots) {
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = res_config(l, std::min(l.shots, s0 + nb - s), st, at);
     if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
     cudaLaunchKernelEx(&cfg, f, make_grid<float>(e), l.r, make_src(e), make_rec(e), (const float*)e->src,
                        (float*)e->p, (float*)e->u, (float*)e->w, (float*)e->seis_t,
-                       store ? (float*)e->strips : (float*)nullptr, lo, hi, s);
+                       store && !save ? (float*)e->strips : (float*)nullptr,
+                       save ? (float4*)e->strips : (float4*)nullptr, lo, hi, s);
     if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
   }
 }
@@ -216,7 +236,7 @@ inline void res_forward(swit_engine* e, const ResLoop& l, bool store, int s0, in
 inline void res_backward(swit_engine* e, const ResLoop& l, int s0, int nb, cudaStream_t st, int hi, int lo,
                          std::vector<cudaEvent_t>* ev = nullptr) {
   if (lo > hi) return;
-  const ResBwdFn f = res_inst(true, l).b;
+  const ResBwdFn f = res_inst(kResLoopBwd, l).b;
   for (int s = s0; s < s0 + nb; s += l.shots) {
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = res_config(l, std::min(l.shots, s0 + nb - s), st, at);
@@ -226,6 +246,17 @@ inline void res_backward(swit_engine* e, const ResLoop& l, int s0, int nb, cudaS
                        (float*)e->ue, (float*)e->we, (float*)e->dg, (float*)e->dfw, (float*)e->dbk,
                        (const float*)e->strips, hi, lo, s);
     if (ev) cudaEventRecord(ev->emplace_back(res_event()), st);
+  }
+}
+
+inline void res_xadj(swit_engine* e, const ResLoop& l, const XAdj<float>& x, int s0, int nb, cudaStream_t st, int hi,
+                     int lo) {
+  if (lo > hi) return;
+  const ResXadjFn f = res_inst(kResLoopXadj, l).x;
+  for (int s = s0; s < s0 + nb; s += l.shots) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = res_config(l, std::min(l.shots, s0 + nb - s), st, at);
+    cudaLaunchKernelEx(&cfg, f, make_grid<float>(e), l.r, make_src(e), make_rec(e), x, hi, lo, s);
   }
 }
 

@@ -100,13 +100,35 @@ def test_checkpointed_segments_match_oracle(every, monkeypatch):
             np.testing.assert_array_equal(a, want[k], err_msg=k)
 
 
+@pytest.mark.parametrize("shape,tiles,every", [(a, t, 0) for a, t in SHAPES if "comp" not in a] +
+                         [(dict(), 2, k) for k in (32, 50, 139, 140)])
+def test_exact_adjoint_matches_oracle(shape, tiles, every, monkeypatch):
+    s, pb = problem(**shape)
+    src, rho = s.source(), s.rho(s.vp_true)
+    adj = np.random.default_rng(tiles).standard_normal((pb.ns, pb.ngmax, s.nt)).astype(np.float32)
+    want = O.exact(pb, s.vp_true, rho, src, adj)
+    split(monkeypatch, tiles)
+    with Engine(**s.engine_args(), adjoint="exact", checkpoint_every=every) as e:
+        assert e.query()["kernel"] == "resident"
+        e.set_model(s.vp_true, rho)
+        seis = e.forward(src, save_boundary=True)
+        first = e.backward_exact(adj)
+        again = e.backward_exact(adj)
+        e.check()
+    np.testing.assert_array_equal(seis, want["seis"])
+    for got in (first, again):
+        np.testing.assert_array_equal(got[0], want["g"])
+        np.testing.assert_array_equal(got[1], want["gsrc"])
+
+
 def test_routes():
     """What the resident loops do not take stays on the step kernels."""
     s, _ = problem()
     for opts, kernel in ((dict(), "resident"), (dict(kernel="vec"), "vec"), (dict(shots_per_batch=1), "vec"),
                          (dict(precision="fp64"), "vec"), (dict(path="plain"), "vec"), (dict(graph_branches=2), "vec"),
                          (dict(block_x=8), "vec"), (dict(checkpoint_every=31), "vec"),
-                         (dict(receiver_component="vx"), "vec"), (dict(adjoint="exact"), "vec")):
+                         (dict(receiver_component="vx"), "vec"), (dict(adjoint="exact"), "resident"),
+                         (dict(adjoint="exact", receiver_component="vz"), "vec")):
         with Engine(**s.engine_args(), **opts) as e:
             assert e.query()["kernel"] == kernel, opts
 
