@@ -121,15 +121,18 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
 }
 
 // Estimated microseconds of one time step of a launch whose fullest SM holds `bpsm` blocks, fitted to
-// measured steps (GB300, 32 to 512 threads per block): a fixed part, the dependent chain of a step
-// (updates, barriers, halo), and a part by the warps that share the SM.  A band of a single column tile
-// exchanges both its edges in the same threads; a shot in one band exchanges nothing.
+// measured steps (GB300, 11 grids of 60x40 to 700x40 and 401x151 in bands of 1 to 10 column tiles, 1 to 15
+// warps per block): a fixed part, the dependent chain of a step (updates, barriers, halo), and a part by the
+// warps that share the SM.  Bands of one column tile exchange both edges in the same threads, and in bands of
+// two every thread has an edge (forward of 101x51: 2.00 us with one tile, 2.06 with two, 1.64 with three);
+// a shot in one band exchanges nothing.  The reverse loop's 128-register instance pays for its spills.
 inline double res_step_us(const ResPlan& r, ResKind kind, int maxt, int bpsm, int tiles) {
   const double warps = bpsm * ((r.nA + r.nR) / 32);
-  const double t = kind == kResLoopXadj  ? 2.0 + 0.12 * warps
-                   : kind == kResLoopFwd ? 1.55 + 0.09 * warps
-                                         : 2.1 + (maxt > 384 ? 0.15 : 0.085) * warps;
-  return t + (r.C > 1 ? (tiles == 1 ? 0.45 : 0.0) : -0.3);
+  const double edge[3][2] = {{0.40, 0.33}, {0.50, 0.20}, {0.50, 0.37}};
+  const double t = kind == kResLoopFwd   ? 1.5 + 0.09 * warps
+                   : kind == kResLoopBwd ? 1.95 + (maxt > 384 ? 0.23 : 0.095) * warps
+                                         : 1.85 + 0.11 * warps;
+  return t + (r.C == 1 ? -0.3 : (tiles <= 2 ? edge[kind][tiles - 1] : 0.0));
 }
 
 // The fastest split by estimate among those whose blocks are co-resident.
