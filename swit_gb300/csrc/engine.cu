@@ -2200,8 +2200,9 @@ int swit_create(const swit_desc* d, swit_engine** out) {
     return fail(SWIT_E_ARG, "vx / vz receivers run on the walk or vec kernels (kernel_variant 0, 2 or 3)");
   }
   e->rcomp = d->receiver_component;
-  // the strip buffer holds D of each step, in the fields' layout or by 4 x 4 tiles from row fs-1 (resident loops)
-  if (e->exact) e->SL = std::max(e->NX * e->LD, round_up(e->NX, 4) * round_up(e->NZ - e->fs + 2, 4));
+  // the strip buffer holds D of each step, in the fields' layout or by columns of row tiles from row fs-1 (resident
+  // loops: whole tiles of up to 8 columns)
+  if (e->exact) e->SL = std::max(e->NX * e->LD, round_up(e->NX, 8) * round_up(e->NZ - e->fs + 2, 4));
   if (e->variant == 2) {
     e->bx = d->block_x > 0 ? d->block_x : 8;  // columns per tile
     if (e->bx < 2 || e->bx > 256) {

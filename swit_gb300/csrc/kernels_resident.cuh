@@ -71,6 +71,7 @@ struct ResPlan {
   int W;         // columns of the widest band
   int ns;        // slots: (tiles of the widest band + 2) nq
   int jz;        // row nz within its tile
+  int nside;     // side arrays a band may hold: 6, or the 3 of one side
   float negz;    // -0 (see f2)
   unsigned wait; // polls before a halo wait gives up
   uint4* halo;   // packets: [block][role][side][parity][packet][row tile]
@@ -85,7 +86,7 @@ struct ResPlan {
   int oX;        // column factors, float2 [W]
   int oD;        // adjoint -> reconstruction, [TX] of a slot; stride TX + 1
   int oStage;    // forward: staged rows, [6][W]
-  int oS;        // forward: side columns, [6][nq]
+  int oS;        // forward: side columns, [nside][nq]
   int oEnt;      // receiver entries
   int oList;     // values moved every step, int2
   int oBox, box; // reverse: inputs of a step (strips, side columns, adjoint sources), [2 steps][box]
@@ -326,7 +327,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 // adds without damping, has factor 1 and negated coefficients: the same values).
 //
 // p from u (x-neighbours in the edge arrays) and w.
-// SAVE: D of the tile to save[column of the tile * (column tiles of the shot) nq].
+// SAVE: D of the tile to save[column of the tile * nq].
 template <int TX, bool SIDE, bool SAVE = false>
 __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int tt0, float (&p)[TX][4],
                                        const float (&u)[TX][4], const float (&w)[TX][4], float c1, float c2,
@@ -364,7 +365,7 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
       sub_if(bit_at(T.f, kP + j), p[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * p[c][j], a[j] * D);
       d[j] = D;
     }
-    if constexpr (SAVE) stg4_if(T.f & kLive, save + c * r.nt_tiles * r.nq, d);
+    if constexpr (SAVE) stg4_if(T.f & kLive, save + c * r.nq, d);
   }
 }
 
@@ -877,6 +878,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   // Traces and strips: the tiles that hold recorded rows stage whole columns in shared memory at the
   // end of a step -- p, u, w at the free surface, p at row nz, p and w at row nz - 1, the side columns --
   // and the block writes the values out by its list in the next step, while its halo is under way.
+  auto side_at = [&](int a) { return a < 3 ? a : a - 6 + r.nside; };
   {
     const StripOff o = strip_offsets(g.nx, g.nz);
     const int jx0 = tt0 * TX + 1 - L;
@@ -902,7 +904,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         const int ix = q < 3 ? (q == 1 ? L + 2 : L + 1) : (q == 3 ? NX - L : NX - L - 1);
         if (ix > tt0 * TX && ix <= (tt0 + n) * TX)
           list_append(r, s_cnt + 1, g.nz,
-                      [&](int i) { return make_int2(4 * (r.oS + q * nq) + i + 1, o.S0 + q * g.nz + i); });
+                      [&](int i) { return make_int2(4 * (r.oS + side_at(q) * nq) + i + 1, o.S0 + q * g.nz + i); });
       }
     }
   }
@@ -922,8 +924,8 @@ __global__ void __launch_bounds__(MAXT, 1)
         const int ix = T.ix0 + c;
         // with nx >= 8 the four columns are distinct
         const int a = ix == L + 1 ? 0 : (ix == L + 2 ? 1 : (ix == NX - L ? 3 : (ix == NX - L - 1 ? 4 : -1)));
-        if (a >= 0) res_sm[r.oS + a * nq + T.k] = mk4(p[c]);
-        if (a == 0 || a == 4) res_sm[r.oS + (a == 0 ? 2 : 5) * nq + T.k] = mk4(u[c]);
+        if (a >= 0) res_sm[r.oS + side_at(a) * nq + T.k] = mk4(p[c]);
+        if (a == 0 || a == 4) res_sm[r.oS + side_at(a == 0 ? 2 : 5) * nq + T.k] = mk4(u[c]);
       }
     }
   };
@@ -944,7 +946,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     // ---- pressure phase
     float4* save = nullptr;
     if constexpr (SAVE)
-      save = dsave + ((size_t)opaque(s) * g.snt + (it - g.sit0)) * (g.SL / 4) + (T.ix0 - 1) / TX * nq + T.k;
+      save = dsave + ((size_t)opaque(s) * g.snt + (it - g.sit0)) * (g.SL / 4) + (T.ix0 - 1) * nq + T.k;
     if (T.f & kSide)
       tile_p<TX, true, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
     else

@@ -200,9 +200,9 @@ __device__ __forceinline__ void xedge_recv(const Tile<TX>& T, const ResPlan& r, 
   }
 }
 
-// Steps it1 .. it0 of shots shot0 + block / C.  D of a step: float4 [column of a tile][column tile of the
-// shot][row tile], as the forward loop stored it; a thread fetches its own a step ahead (16 bytes per column
-// and thread, coalesced).  384 threads of 168 registers, for four 16-value arrays.
+// Steps it1 .. it0 of shots shot0 + block / C.  D of a step: float4 [column][row tile], as the
+// forward loop stored it (whatever its columns per thread); a thread fetches its own a step ahead, 16 bytes
+// per column, consecutive in a warp.  384 threads of 168 registers, for four 16-value arrays.
 //
 // Bound by the dependent chain of a step, and on a full device by issue.  10 shots 241x121, per step, against
 // the kernels of kernels_exact.cuh: forward keeping D 2.15, reverse 2.63 us, together 18.8 -> 4.8 us (gradient
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   __syncthreads();
   const int nrec = s_cnt[0];
   const float4* dsave = reinterpret_cast<const float4*>(x.dsave);
-  const int dcol = r.nt_tiles * nq, dat = (T.ix0 - 1) / TX * nq + T.k;
+  const int dat = (T.ix0 - 1) * nq + T.k;
   // inputs of a step: its adjoint sources (entries without a receiver, the padding of a tile's, repeat
   // receiver 0: never read) and D
   auto prefetch = [&](int it) {
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     const float4* d = dsave + (so * g.snt + (it - g.sit0)) * (g.SL / 4) + dat;
     if (T.f & kLive)
 #pragma unroll
-      for (int c = 0; c < TX; ++c) cp16(res_sm + r.oD + c * r.nA + tid, d + c * dcol);
+      for (int c = 0; c < TX; ++c) cp16(res_sm + r.oD + c * r.nA + tid, d + c * nq);
   };
   prefetch(it1);
   cp_wait();

@@ -31,11 +31,12 @@ struct ResInst {
   const void* any() const { return f ? (const void*)f : (b ? (const void*)b : (const void*)x); }
 };
 inline const ResInst* res_instances(ResKind kind, int& n) {
-  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512, false>, k_fwd_res<4, 512, true>, nullptr, nullptr}};
+  static const ResInst F[] = {{4, 512, k_fwd_res<4, 512, false>, k_fwd_res<4, 512, true>, nullptr, nullptr},
+                              {8, 384, k_fwd_res<8, 384, false>, k_fwd_res<8, 384, true>, nullptr, nullptr}};
   static const ResInst B[] = {{4, 512, nullptr, nullptr, k_bwd_res<4, 512>, nullptr},
                               {4, 384, nullptr, nullptr, k_bwd_res<4, 384>, nullptr}};
   static const ResInst X[] = {{4, 384, nullptr, nullptr, nullptr, k_xadj_res<4, 384>}};
-  n = kind == kResLoopBwd ? 2 : 1;
+  n = kind == kResLoopXadj ? 1 : 2;
   return kind == kResLoopFwd ? F : (kind == kResLoopBwd ? B : X);
 }
 
@@ -50,6 +51,8 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
   r.W = widest * tx;
   r.m0 = e->L / tx;
   r.m1 = (e->L + e->nx - 1) / tx;
+  // a band reaches the strip columns of both sides only if it is nearly as wide as the interior
+  r.nside = bwd || r.W + 8 >= e->nx ? 6 : 3;
   if (bwd) {
     r.kr = (e->fs - 2 + 3) / 4;  // rows from fs-1-4 kr <= 1
     r.nq = (e->NZ - (e->fs - 1 - 4 * r.kr) + 1 + 3) / 4;
@@ -112,9 +115,9 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
     r.oEnt = take(1 + r.ent_cap / 2);
   } else {
     r.oStage = take(6 * r.W);
-    r.oS = take(6 * r.nq);
+    r.oS = take(r.nside * r.nq);
     r.oEnt = take(1 + (2 * r.ent_cap + r.W + 3) / 4);  // counters, receivers, codes, columns
-    r.oList = take((10 * r.W + 6 * e->nz + 1) / 2);
+    r.oList = take((10 * r.W + r.nside * e->nz + 1) / 2);
   }
   r.smem = 16 * o;
   return r;
@@ -125,11 +128,14 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
 // warps per block): a fixed part, the dependent chain of a step (updates, barriers, halo), and a part by the
 // warps that share the SM.  Bands of one column tile exchange both edges in the same threads, and in bands of
 // two every thread has an edge (forward of 101x51: 2.00 us with one tile, 2.06 with two, 1.64 with three);
-// a shot in one band exchanges nothing.  The reverse loop's 128-register instance pays for its spills.
+// a shot in one band exchanges nothing.  The reverse loop's 128-register instance pays for its spills; the
+// forward's with 8 columns per thread holds half as many points again per SM and is taken where that saves
+// launches (10 shots 801x301: 9.7 against 11.0 us per step in 2 and 4 launches; 49 shots 481x141: 17.9
+// against 14.2) or nothing else fits (2001x601).
 inline double res_step_us(const ResPlan& r, ResKind kind, int maxt, int bpsm, int tiles) {
   const double warps = bpsm * ((r.nA + r.nR) / 32);
   const double edge[3][2] = {{0.40, 0.33}, {0.50, 0.20}, {0.50, 0.37}};
-  const double t = kind == kResLoopFwd   ? 1.5 + 0.09 * warps
+  const double t = kind == kResLoopFwd   ? 1.5 + (maxt < 512 ? 0.28 : 0.09) * warps
                    : kind == kResLoopBwd ? 1.95 + (maxt > 384 ? 0.23 : 0.095) * warps
                                          : 1.85 + 0.11 * warps;
   return t + (r.C == 1 ? -0.3 : (tiles <= 2 ? edge[kind][tiles - 1] : 0.0));
@@ -144,14 +150,17 @@ inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
     return;
   int want = 0;  // column tiles per band instead of the estimate's choice, e.g. to test a split
   if (const char* v = std::getenv(kind != kResLoopFwd ? "SWIT_RES_BWD_TILES" : "SWIT_RES_FWD_TILES")) want = std::atoi(v);
+  int cols = 0;  // columns per thread, likewise
+  if (const char* v = std::getenv("SWIT_RES_FWD_COLS")) cols = kind == kResLoopFwd ? std::atoi(v) : 0;
   int ninst = 0;
   const ResInst* I = res_instances(kind, ninst);
   double best = 0.0;
   for (int i = 0; i < ninst; ++i) {
+    if (cols && I[i].tx != cols) continue;
     const int all = (e->NX + I[i].tx - 1) / I[i].tx;
     int lastC = -1;
     for (int tiles = 1; tiles <= all; ++tiles) {
-      if (want && tiles != want) continue;
+      if (want && tiles != std::min(want, all)) continue;
       ResPlan r = res_plan(e, kind, I[i].tx, tiles);
       if (r.C == lastC) continue;
       lastC = r.C;

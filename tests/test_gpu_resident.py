@@ -7,7 +7,8 @@ illuminations.  The sizes sit where a split can go wrong: bands of one, two and
 three 4-column tiles and a shot in one band, grids whose last tile has 1 to 4
 columns, every alignment of the free surface and of the bottom row to the 4-row
 tiles, the smallest grid, columns of several warps, scattered and coinciding
-receivers.  SWIT_RES_FWD_TILES / SWIT_RES_BWD_TILES set the band width.
+receivers.  SWIT_RES_FWD_TILES / SWIT_RES_BWD_TILES set the band width,
+SWIT_RES_FWD_COLS the forward's columns per thread (4 or 8).
 """
 import numpy as np
 import pytest
@@ -45,12 +46,14 @@ SHAPES = ([(dict(nx=37, nz=28, npml=n), t) for n in (8, 9, 10, 11) for t in (1, 
            (dict(comp="vx"), 2), (dict(comp="vz"), 2)])
 
 
+@pytest.mark.parametrize("cols", [4, 8])
 @pytest.mark.parametrize("shape,tiles", SHAPES)
-def test_forward_matches_oracle(shape, tiles, monkeypatch):
+def test_forward_matches_oracle(shape, tiles, cols, monkeypatch):
     s, pb = problem(**shape)
     src, rho = s.source(), s.rho(s.vp_true)
     ref = O.forward(pb, s.vp_true, rho, src, store=True)
     split(monkeypatch, tiles)
+    monkeypatch.setenv("SWIT_RES_FWD_COLS", str(cols))
     with Engine(**s.engine_args(), receiver_component=shape.get("comp", "p")) as e:
         e.set_model(s.vp_true, rho)
         plain = e.forward(src, save_boundary=False)
@@ -100,14 +103,16 @@ def test_checkpointed_segments_match_oracle(every, monkeypatch):
             np.testing.assert_array_equal(a, want[k], err_msg=k)
 
 
+@pytest.mark.parametrize("cols", [4, 8])
 @pytest.mark.parametrize("shape,tiles,every", [(a, t, 0) for a, t in SHAPES if "comp" not in a] +
                          [(dict(), 2, k) for k in (32, 50, 139, 140)])
-def test_exact_adjoint_matches_oracle(shape, tiles, every, monkeypatch):
+def test_exact_adjoint_matches_oracle(shape, tiles, every, cols, monkeypatch):
     s, pb = problem(**shape)
     src, rho = s.source(), s.rho(s.vp_true)
     adj = np.random.default_rng(tiles).standard_normal((pb.ns, pb.ngmax, s.nt)).astype(np.float32)
     want = O.exact(pb, s.vp_true, rho, src, adj)
     split(monkeypatch, tiles)
+    monkeypatch.setenv("SWIT_RES_FWD_COLS", str(cols))
     with Engine(**s.engine_args(), adjoint="exact", checkpoint_every=every) as e:
         assert e.query()["kernel"] == "resident"
         e.set_model(s.vp_true, rho)
