@@ -2091,7 +2091,10 @@ const char* swit_last_error(void) { return g_err.c_str(); }
 // 0.7 L2 / state, branches br (3 unless given), batches k = br * ceil(ns / T)
 // (a multiple of br, so the branches get the same number of launches) and
 // ceil(ns / k) shots per batch.  At 481x141 (npml 40) on GB300: 28 shots in
-// flight, 6 batches of 9 on 3 branches.
+// flight, 6 batches of 9 on 3 branches.  Where fewer shots fit, fewer branches
+// run: their state would push each other's out of L2 (reverse step of 3 shots
+// 2001x601: 60.9 us on 3 branches, 53.7 on 2, 58.8 on 1; of 2 shots 3001x801:
+// 85.1 on 2, 81.5 on 1).
 void auto_batches(swit_engine* e, int branches) {
   int dev = 0, l2 = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
@@ -2101,8 +2104,9 @@ void auto_batches(swit_engine* e, int branches) {
   // fields and imaging sums on the interior; the walk kernels keep two sets
   const double state = e->variant == 2 ? (6.0 * e->NX * e->NZ + 9.0 * e->nx * e->nz) * e->esz
                                        : (3.0 * e->NX * e->NZ + 6.0 * e->nx * e->nz) * e->esz;
-  const int inflight = std::max(1, (int)(0.7 * l2 / state));
-  const int br = std::max(1, std::min(branches ? branches : 3, e->ns));
+  const double fit = 0.7 * l2 / state;
+  const int inflight = std::max(1, (int)fit);
+  const int br = std::max(1, std::min(branches ? branches : std::min(3, (int)(fit + 0.5)), e->ns));
   const int per_branch = std::max(1, inflight / br);
   const int rounds = (e->ns + br * per_branch - 1) / (br * per_branch);
   // and at most about 1 M kernel nodes per captured loop (grids whose state
