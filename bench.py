@@ -108,6 +108,14 @@ def kernel_bytes_per_shot(nx, nz, npml, ng, nt):
     return step
 
 
+def loop_ops_per_shot(nx, nz, npml, nt):
+    """FP32 operations of one resident time loop per shot (no FMA, so one per lane and instruction slot): 28
+    per PML point for the three updates, and in the reverse loop 28 + 3 per PML point of the adjoint and 25 + 4
+    per interior point of the reconstruction and the image."""
+    npts, nint = (nx + 2 * npml) * (nz + npml), nx * nz
+    return {"fwd_loop": (nt - 1) * 28 * npts, "bwd_loop": (nt - 1) * (31 * npts + 29 * nint)}
+
+
 def measured_peak():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -488,7 +496,8 @@ def run_mine(args):
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": workload_config(sv, per_rank),
-            "engine": {"path": "batched, CUDA graph", "kernel": q["kernel"], "shots_per_launch": q["shots_per_batch"],
+            "engine": {"path": "whole time loops, one cooperative launch per group of shots"
+                       if q["kernel"] == "resident" else "batched, CUDA graph", "kernel": q["kernel"], "shots_per_launch": q["shots_per_batch"],
                        "block_x": q["block_x"], "graph_branches": q["graph_branches"], "adjoint": args.adjoint,
                        "parallelism": "shots" + ("" if world == 1 else " x%d ranks" % world)},
             "autotune": {"trial_steps": 48, "candidates": tuned} if tuned else None,
@@ -514,7 +523,7 @@ def run_mine(args):
         kb = kernel_bytes_per_shot(sv.nx, sv.nz, sv.npml, sv.ng, sv.nt)
         nbatch = -(-per_rank // q["shots_per_batch"])
         shots_launch = per_rank / nbatch  # mean shots per launch (the last batch may be smaller)
-        vec = q["kernel"] == "vec"
+        vec, res = q["kernel"] == "vec", q["kernel"] == "resident"
         kern = {}
         for k, v in prof.items():
             per_step = v["mean_ms"] * (nbatch if vec else v["launches"] / (sv.nt - 1))
@@ -523,6 +532,8 @@ def run_mine(args):
         for k in kern:
             kern[k]["share"] = kern[k]["ms_per_gradient"] / tot
         top = max(kern, key=lambda k: kern[k]["ms_per_gradient"])
+        if res:
+            shots_launch = per_rank / prof[top]["launches"]
         alg = kb[top] * shots_launch
         achieved = alg / (prof[top]["mean_ms"] / 1000.0) / 1e9
         l2 = l2_bandwidth()
@@ -543,10 +554,24 @@ def run_mine(args):
                                       "events around every launch",
                             "kernels": kern, "kernels_ms_per_gradient": tot,
                             "ms_per_step": ms_per_step}
+        if res:
+            # the fields stay in registers for the whole loop: what is left to bound it is FP32 issue, one
+            # operation per lane and cycle at the clock seen during the timed region
+            props = torch.cuda.get_device_properties(local)
+            mhz = (clk or {}).get("sm_mhz") or (clk or {}).get("sm_max_mhz") or 2070
+            ops = loop_ops_per_shot(sv.nx, sv.nz, sv.npml, sv.nt)[top] * shots_launch
+            opeak = props.multi_processor_count * 128 * mhz * 1e6 / 1e9
+            oach = ops / (prof[top]["mean_ms"] / 1000.0) / 1e9
+            line["roofline"].update(
+                bound="fp32 issue", achieved=oach, peak=opeak, unit="GFLOP/s", frac=oach / opeak,
+                peak_kind="%d SMs x 128 lanes x %d MHz, no FMA" % (props.multi_processor_count, int(mhz)),
+                algorithmic_ops_per_launch=ops, hbm_peak_gbs=peak,
+                step_kernel_bytes_gbs=achieved, l2_frac=None,
+                bytes_note="step_kernel_bytes_gbs: what kernels of one step each would move through L2 in this time")
         # plain one-shot-per-launch path on a bounded sample
         nplain = min(4, per_rank)
         pe = Engine(sv.nx, sv.nz, sv.npml, sv.nt, sv.dx, sv.dt, src_xz[:nplain], rec_xz[:nplain], path="plain",
-                    kernel=q["kernel"], block_x=q["block_x"])
+                    kernel="vec" if res else q["kernel"], block_x=q["block_x"])
         pe.set_model(sv.vp_init, rho)
         src_p, obs_p = src_d[:nplain].contiguous(), obs_d[:nplain].contiguous()
         pe.gradient_l2(src_p, obs_p)

@@ -1,8 +1,8 @@
 """Launch-configuration autotuner.
 
 Times a short Waveform-gradient run (the full geometry and shot count, a few
-dozen time steps) for each candidate (shots per launch, concurrent graph
-branches of the vec kernels) and returns the fastest.  Every candidate computes bit-identical
+dozen time steps) for each candidate (the default kernels; shots per launch and
+concurrent graph branches of the vec kernels) and returns the fastest.  Every candidate computes bit-identical
 results, so the choice only affects speed.  Results are cached per process
 by problem shape.
 """
@@ -43,9 +43,10 @@ def tune(nx, nz, npml, dx, dt, src_xz, rec_xz, vp, rho, free_surface=1, trial_st
     key = (nx, nz, npml, ns, rec_xz.shape[-2], trial_steps, free_surface, adjoint)
     if key in _cache and cands is None:
         return _cache[key]
-    cands = cands or candidates(ns)
-    if adjoint == "exact":  # the exact adjoint runs on the vec kernels
-        cands = [c for c in cands if c["kernel"] == "vec"]
+    # the default kernels (resident time loops where they fit) beside the vec launch shapes
+    cands = cands or [dict(kernel="auto", block_x=0, shots_per_batch=0, graph_branches=0)] + candidates(ns)
+    if adjoint == "exact":  # the exact adjoint runs on the default or the vec kernels
+        cands = [c for c in cands if c["kernel"] in ("auto", "vec")]
     nt = trial_steps
     rng = np.random.default_rng(0)
     src = torch.from_numpy(rng.standard_normal((ns, nt)).astype(np.float32)).cuda()
