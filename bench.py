@@ -748,7 +748,7 @@ def run_correlation(args):
     ckpt = int(args.checkpoint) if args.checkpoint != "auto" else 0
     opts = dict(shots_per_batch=args.batch, block_x=args.block_x, graph_branches=args.branches, adjoint=args.adjoint,
                 checkpoint_every=ckpt)
-    eng = Engine(**sv.engine_args(), kernel="vec" if args.kernel == "auto" else args.kernel, **opts)
+    eng = Engine(**sv.engine_args(), kernel=args.kernel, **opts)
     q = eng.query()
     rho = torch.from_numpy(sv.rho(sv.vp_true)).cuda()
     src = torch.from_numpy(sv.source()).cuda()

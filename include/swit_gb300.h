@@ -113,7 +113,8 @@ typedef struct swit_desc {
   int32_t graph_branches;   /* batched path: the shot batches' step chains form
                                this many concurrent branches of the captured
                                graphs (batch b on branch b mod graph_branches);
-                               0 = automatic (3 with automatic shots_per_batch,
+                               0 = automatic (with automatic shots_per_batch as
+                               many as shots whose state fits in L2, at most 3;
                                else 2), at most 4                               */
   int32_t adjoint_mode;     /* 0 = fd2dmpi's adjoint (boundary strips, reverse
                                reconstruction, continuous-adjoint imaging:
@@ -208,7 +209,8 @@ int swit_l2_bandwidth(int64_t bytes, int32_t reps, double* gbs, void* stream);
  * four add up to about the loop's.  Other engines launch every kernel of a
  * forward and reverse loop with an event pair around it.  With the walk
  * variant, [0] is the forward step kernel, [2] the reverse step kernel and [1],
- * [3] are unused (0 launches).  Leaves the wavefields undefined until the next
+ * [3] are unused (0 launches); with resident loops likewise, [0] being a forward
+ * and [2] a reverse time loop of a group of shots.  Leaves the wavefields undefined until the next
  * forward run; synchronises the stream. */
 int swit_profile_kernels(swit_engine* e, int32_t launches[4], double mean_ms[4], void* stream);
 
@@ -261,8 +263,9 @@ int swit_backward_exact(swit_engine* e, const float* adj, void* grad, void* src_
                         void* stream);
 
 /* Waits for `stream` and reports whether any kernel of the engine gave up
- * waiting for the copies it stages into shared memory (band variant: every such
- * wait is bounded, and a block that times out skips its update).  Returns
+ * waiting, for the copies it stages into shared memory (band variant) or for a
+ * neighbour band's halo (resident loops): every such wait is bounded; what the
+ * engine computed after one that ran out is invalid.  Returns
  * SWIT_E_TIMEOUT once for such an event, then clears it.  No counterpart in the
  * reference, whose CPU loops have no asynchronous copies. */
 int swit_check(swit_engine* e, void* stream);
@@ -277,7 +280,8 @@ int swit_misfit_l2(swit_engine* e, const float* src, const float* obs, double* m
  * A multi-instance engine holds n regular engines (one swit_desc each: FP32,
  * batched path, vec kernels, boundary saving; grids, shot counts and nt may all
  * differ) and steps them together: the (instance, shot) pairs are grouped
- * into L2-sized waves (an instance's own shots, or several small instances),
+ * into L2-sized waves (an instance's own shots, or several small instances;
+ * instances whose time loops fit the device as resident loops run those instead),
  * and per wave each time step launches the phase kernels once over every pair
  * still running; the waves run on concurrent branches, and a call runs only
  * the waves holding a switched-on instance (swit_multi_misfit_l2's `active`).

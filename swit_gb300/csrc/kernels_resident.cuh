@@ -38,7 +38,7 @@
 //
 // Update ranges.  Every point of a tile is updated; what the reference never
 // updates is put right afterwards: the few of those values that a later update
-// reads hold their initial zero (fix_* below), and everything the
+// reads hold their initial zero (predicated rows, zero_cols), and everything the
 // reconstruction does not update is re-inserted from the strips.
 //
 // Registers and instructions are what limits these kernels, so a thread keeps
@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   // Traces and strips: the tiles that hold recorded rows stage whole columns in shared memory at the
   // end of a step -- p, u, w at the free surface, p at row nz, p and w at row nz - 1, the side columns --
   // and the block writes the values out by its list in the next step, while its halo is under way.
-  auto side_at = [&](int a) { return a < 3 ? a : a - 6 + r.nside; };
+  auto side_at = [&](int a) { return TX == 4 || a < 3 ? a : a - 6 + r.nside; };
   {
     const StripOff o = strip_offsets(g.nx, g.nz);
     const int jx0 = tt0 * TX + 1 - L;

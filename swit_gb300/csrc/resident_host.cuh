@@ -51,8 +51,9 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
   r.W = widest * tx;
   r.m0 = e->L / tx;
   r.m1 = (e->L + e->nx - 1) / tx;
-  // a band reaches the strip columns of both sides only if it is nearly as wide as the interior
-  r.nside = bwd || r.W + 8 >= e->nx ? 6 : 3;
+  // a band reaches the strip columns of both sides only if it is nearly as wide as the interior; with 4 columns
+  // per thread there is room for both, and a constant index (481x141: 14.1 against 14.3 us per step)
+  r.nside = tx == 4 || r.W + 8 >= e->nx ? 6 : 3;
   if (bwd) {
     r.kr = (e->fs - 2 + 3) / 4;  // rows from fs-1-4 kr <= 1
     r.nq = (e->NZ - (e->fs - 1 - 4 * r.kr) + 1 + 3) / 4;

@@ -138,6 +138,30 @@ def test_routes():
             assert e.query()["kernel"] == kernel, opts
 
 
+@pytest.mark.parametrize("bad", [np.inf, np.nan, np.finfo(np.float32).max])
+def test_values_that_are_not_finite_spread_as_in_the_step_kernels(bad, monkeypatch):
+    """What a tile computes beyond the update ranges never reaches a value inside them."""
+    s, pb = problem(ns=3)
+    src = s.source().copy()
+    src[1, 40] = bad
+    rho, out = s.rho(s.vp_true), []
+    split(monkeypatch, 2)
+    for kernel in ("auto", "vec"):
+        with Engine(**s.engine_args(), kernel=kernel) as e:
+            e.set_model(s.vp_true, rho)
+            seis = e.forward(src, save_boundary=True)
+            adj = seis.copy()
+            adj[2, 3, 90] = bad
+            out.append([seis, *e.backward(adj)])
+        with Engine(**s.engine_args(), kernel=kernel, adjoint="exact") as e:
+            e.set_model(s.vp_true, rho)
+            e.forward(src, save_boundary=True)
+            out[-1] += e.backward_exact(adj)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert np.isfinite(out[0][0][[0, 2]]).all()
+
+
 def test_halo_timeout_is_reported_and_the_context_stays_usable(monkeypatch):
     """With a poll limit of 0 every halo wait gives up at its first miss, records
     it in the engine's error word and goes on without waiting: the call with host
