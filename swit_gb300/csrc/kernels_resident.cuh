@@ -33,8 +33,11 @@
 // monotone, so a factor 1 - kappa is the smaller of a column's and a row's:
 // p: min(fx, fz), u: min(fxu, fz), w: min(fx, fzw), where fxu (fzw) averages two
 // neighbouring columns (rows) -- neighbouring cell numbers differ by one, so
-// iX is never strictly between those of two rows.  Away from the sides fx = 1
-// and the minimum is skipped.
+// iX is never strictly between those of two rows.  Tiles away from the sides,
+// where fx = 1, take the minimum all the same: a second copy of the updates
+// without it cost more in the instruction cache than the minimum does (49 shots
+// 481x141: 14.1 against 13.2 us per forward step, 37.4 against 35.2 per reverse
+// step).
 //
 // Update ranges.  Every point of a tile is updated; what the reference never
 // updates is put right afterwards: the few of those values that a later update
@@ -236,11 +239,10 @@ __device__ __forceinline__ void cp4(void* dst, const void* src) {
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// Flags of a thread's tile.  kSide and kRare are uniform over the warp.
+// Flags of a thread's tile.  kRare is uniform over the warp.
 enum : unsigned {
   kLive = 1u << 0,   // holds a tile
   kAdj = 1u << 1,    // adjoint role (reverse kernel)
-  kSide = 1u << 2,   // the warp touches the side layers: column factors
   kRare = 1u << 3,   // the warp has band edges, columns to zero, side strips, the source or scattered receivers
   kEnds = 1u << 4,   // the tile has columns to zero
   kLeft = 1u << 5,   // at the band's left edge, and a neighbour band exists
@@ -324,11 +326,12 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 }
 
 // The updates of a tile, the same code for every role: f := factor f - coef D (the reconstruction, which
-// adds without damping, has factor 1 and negated coefficients: the same values).
+// adds without damping, has row factor 1 and negated coefficients: the same values; its last column's u, the
+// one interior value with a column factor below 1, is never read).
 //
 // p from u (x-neighbours in the edge arrays) and w.
 // SAVE: D of the tile to save[column of the tile * nq].
-template <int TX, bool SIDE, bool SAVE = false>
+template <int TX, bool SAVE = false>
 __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int tt0, float (&p)[TX][4],
                                        const float (&u)[TX][4], const float (&w)[TX][4], float c1, float c2,
                                        float4* save = nullptr) {
@@ -343,9 +346,9 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
   zrow_get<TX>(r, 1, 5, e6);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
-    float a[4], fx = 1.f;
+    float a[4];
     lds4(r.oC + (2 * TX + 1) * threadIdx.x + c, a);
-    if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).x;
+    const float fx = col_factor<TX>(T, r, tt0, c).x;
     float z[7];  // w at rows -2 .. 4
     z[0] = __shfl_up_sync(0xffffffffu, w[c][2], 1);
     z[1] = __shfl_up_sync(0xffffffffu, w[c][3], 1);
@@ -362,7 +365,7 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
       const float l2 = c >= 2 ? u[c >= 2 ? c - 2 : 0][j] : (c == 1 ? um1[j] : um2[j]);
       const float r1 = c + 1 < TX ? u[c + 1 < TX ? c + 1 : 0][j] : up1[j];
       const float D = c1 * (u[c][j] - l1 + z[j + 2] - z[j + 1]) + c2 * (r1 - l2 + z[j + 3] - z[j]);
-      sub_if(bit_at(T.f, kP + j), p[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * p[c][j], a[j] * D);
+      sub_if(bit_at(T.f, kP + j), p[c][j], fminf(fx, fz[j]) * p[c][j], a[j] * D);
       d[j] = D;
     }
     if constexpr (SAVE) stg4_if(T.f & kLive, save + c * r.nq, d);
@@ -370,7 +373,7 @@ __device__ __forceinline__ void tile_p(const Tile<TX>& T, const ResPlan& r, int 
 }
 
 // w from p.
-template <int TX, bool SIDE, bool PACK>
+template <int TX, bool PACK>
 __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int tt0, const float (&p)[TX][4],
                                        float (&w)[TX][4], float c1, float c2) {
   const int lane = threadIdx.x & 31;
@@ -382,9 +385,9 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
   const f2 Z = pk(r.negz, r.negz), C1 = pk(c1, c1), C2 = pk(c2, c2);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
-    float a[4], fx = 1.f;
+    float a[4];
     lds4(r.oC + (2 * TX + 1) * threadIdx.x + TX + c, a);
-    if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).x;
+    const float fx = col_factor<TX>(T, r, tt0, c).x;
     float z[7];  // p at rows -1 .. 5
     z[0] = __shfl_up_sync(0xffffffffu, p[c][3], 1);
     z[5] = __shfl_down_sync(0xffffffffu, p[c][0], 1);
@@ -398,7 +401,7 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float D = c1 * (z[j + 2] - z[j + 1]) + c2 * (z[j + 3] - z[j]);
-        sub_if(bit_at(T.f, kW + j), w[c][j], (SIDE ? fminf(fx, fz[j]) : fz[j]) * w[c][j], a[j] * D);
+        sub_if(bit_at(T.f, kW + j), w[c][j], fminf(fx, fz[j]) * w[c][j], a[j] * D);
       }
     } else {
 #pragma unroll
@@ -406,7 +409,7 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
         const f2 d1 = pk(z[j + 2] - z[j + 1], z[j + 3] - z[j + 2]), d2 = pk(z[j + 3] - z[j], z[j + 4] - z[j + 1]);
         const f2 D = add2(fma2(C1, d1, Z), fma2(C2, d2, Z));
         const f2 S = fma2(pk(a[j], a[j + 1]), D, Z);
-        const f2 F = SIDE ? pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1])) : pk(fz[j], fz[j + 1]);
+        const f2 F = pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1]));
         const f2 Q = fma2(F, pk(w[c][j], w[c][j + 1]), Z);
         float s0, s1, q0, q1;
         upk(S, s0, s1);
@@ -419,7 +422,7 @@ __device__ __forceinline__ void tile_w(const Tile<TX>& T, const ResPlan& r, int 
 }
 
 // u from p (x-neighbours in the edge arrays).
-template <int TX, bool SIDE>
+template <int TX>
 __device__ __forceinline__ void tile_u(const Tile<TX>& T, const ResPlan& r, int tt0, const float (&p)[TX][4],
                                        float (&u)[TX][4], float c1, float c2) {
   float pm1[4], pp1[4], pp2[4], fz[4];
@@ -430,9 +433,9 @@ __device__ __forceinline__ void tile_u(const Tile<TX>& T, const ResPlan& r, int 
   const f2 Z = pk(r.negz, r.negz), M = pk(-1.f, -1.f), C1 = pk(c1, c1), C2 = pk(c2, c2);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
-    float a[4], fx = 1.f;
+    float a[4];
     lds4(r.oC + (2 * TX + 1) * threadIdx.x + TX + c, a);
-    if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).y;
+    const float fx = col_factor<TX>(T, r, tt0, c).y;
 #pragma unroll
     for (int j = 0; j < 4; j += 2) {
       auto P = [&](int k) {
@@ -442,7 +445,7 @@ __device__ __forceinline__ void tile_u(const Tile<TX>& T, const ResPlan& r, int 
       const f2 d1 = fma2(P(c), M, P(c + 1)), d2 = fma2(P(c - 1), M, P(c + 2));
       const f2 D = add2(fma2(C1, d1, Z), fma2(C2, d2, Z));
       const f2 S = fma2(pk(a[j], a[j + 1]), D, Z);
-      const f2 F = SIDE ? pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1])) : pk(fz[j], fz[j + 1]);
+      const f2 F = pk(fminf(fx, fz[j]), fminf(fx, fz[j + 1]));
       const f2 U = fma2(S, M, fma2(F, pk(u[c][j], u[c][j + 1]), Z));
       upk(U, u[c][j], u[c][j + 1]);
     }
@@ -638,11 +641,10 @@ __device__ __forceinline__ void tile_setup(Tile<TX>& T, const Grid<float>& g, co
     f |= 255u << kP;
   } else {
     if (ROLE == kResAdj) f |= kAdj;
-    if (__any_sync(0xffffffffu, strip)) f |= kSide;
     f |= row_bits(iz0, ROLE == kResFwd ? fs + 1 : 3, NZ - 2) << kP | row_bits(iz0, ROLE == kResFwd ? fs : 2, NZ - 2) << kW;
     if (live && (T.ix0 < 3 || T.ix0 + TX - 1 > NX - 2)) f |= kEnds;
   }
-  T.f = live ? f : f & (kAdj | kSide);
+  T.f = live ? f : f & kAdj;
 }
 
 // Ghost tables of an edge thread: coefficient and damping factor of u at the
@@ -894,7 +896,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       } else if (strips && a < 10) {
         // B0, B1 (p), B2 (w); T0, T1, T2 (p), T3, T4 (u), T5 (w): rows fs .. of the top tile
         const int q = a - 1;
-        const int row = q < 3 ? 3 + q : (q < 6 ? 0 : (q < 8 ? 1 : 2));
+        const int row = q < 3 ? (q == 1 && r.jz ? 3 : 3 + q) : (q < 6 ? 0 : (q < 8 ? 1 : 2));
         const int j = q < 1 ? (g.nz & 3) : (q < 3 ? ((g.nz - 1) & 3) : (q < 6 ? q - 2 : (q < 8 ? q - 5 : 1)));
         const int from = 4 * (r.oStage + row * r.W + flo) + j;
         const int to = (q < 3 ? q * g.nx : o.T0 + (q - 3) * g.nx) + jx0 + flo - 1;
@@ -910,13 +912,15 @@ __global__ void __launch_bounds__(MAXT, 1)
   }
   __syncthreads();
   const int nlist = s_cnt[1];
+  // (forward of 49 shots 481x141 without strips, staging p alone: 13.2 -> 12.4 us per step)
   auto stage = [&]() {
     put_cols<TX>(T.f & kTop, r.oStage + xl, p);
+    if (!strips && rec.comp == 0) return;
     put_cols<TX>(T.f & kTop, r.oStage + r.W + xl, u);
     put_cols<TX>(T.f & kTop, r.oStage + 2 * r.W + xl, w);
     if (!strips) return;
     put_cols<TX>(T.f & kB0, r.oStage + 3 * r.W + xl, p);
-    put_cols<TX>(T.f & kB1, r.oStage + 4 * r.W + xl, p);
+    if (r.jz == 0) put_cols<TX>(T.f & kB1, r.oStage + 4 * r.W + xl, p);  // else rows nz-1 and nz share a tile
     put_cols<TX>(T.f & kB1, r.oStage + 5 * r.W + xl, w);
     if ((T.f & (kRare | kStrip)) == (kRare | kStrip)) {
 #pragma unroll
@@ -947,10 +951,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     float4* save = nullptr;
     if constexpr (SAVE)
       save = dsave + ((size_t)opaque(s) * g.snt + (it - g.sit0)) * (g.SL / 4) + (T.ix0 - 1) * nq + T.k;
-    if (T.f & kSide)
-      tile_p<TX, true, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
-    else
-      tile_p<TX, false, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
+    tile_p<TX, SAVE>(T, r, tt0, p, u, w, c1, c2, save);
     if (T.f & kRare) {
       if (T.f & kEnds) zero_cols<TX>(T.ix0, p, 3, NX - 2);
       if (isrc >= 0) {
@@ -965,10 +966,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (it > it0) flush(it - 1);
     __syncthreads();
     // ---- velocity phase
-    if (T.f & kSide)
-      tile_w<TX, true, false>(T, r, tt0, p, w, c1, c2);
-    else
-      tile_w<TX, false, false>(T, r, tt0, p, w, c1, c2);
+    tile_w<TX, false>(T, r, tt0, p, w, c1, c2);
 #pragma unroll
     for (int c = 0; c < TX; ++c) mov_if(T.f & kTopFs, w[c][0], w[c][1]);
     if (T.f & kRare) {
@@ -976,10 +974,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       edge_recv<TX, false>(T, r, 0, r.oG, gu, dead, p, (unsigned)it, c1, c2, h);
     }
     __syncwarp();
-    if (T.f & kSide)
-      tile_u<TX, true>(T, r, tt0, p, u, c1, c2);
-    else
-      tile_u<TX, false>(T, r, tt0, p, u, c1, c2);
+    tile_u<TX>(T, r, tt0, p, u, c1, c2);
     if ((T.f & kRare) && (T.f & kEnds)) zero_cols<TX>(T.ix0, u, 2, NX - 2);
     publish_uw<TX>(T, r, u, w);
     stage();
@@ -1188,10 +1183,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (!(T.f & kAdj) && it < it1) image();
     Halo h;
     edge_issue<TX>(T, r, role, (unsigned)(it + 1), h);
-    if (T.f & kSide)
-      tile_w<TX, true, true>(T, r, tt0, p, w, c1, c2);
-    else
-      tile_w<TX, false, true>(T, r, tt0, p, w, c1, c2);
+    tile_w<TX, true>(T, r, tt0, p, w, c1, c2);
     if (T.f & kAdj) {
       // outside the update range of w both rows are never read
 #pragma unroll
@@ -1216,10 +1208,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       }
     }
     __syncwarp();
-    if (T.f & kSide)
-      tile_u<TX, true>(T, r, tt0, p, u, c1, c2);
-    else
-      tile_u<TX, false>(T, r, tt0, p, u, c1, c2);
+    tile_u<TX>(T, r, tt0, p, u, c1, c2);
     if (T.f & kRare) {
       if (T.f & kEnds) zero_cols<TX>(T.ix0, u, 2, NX - 2);
       if ((T.f & (kStrip | kAdj)) == kStrip) {
@@ -1242,10 +1231,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       add_at<TX, true>(p, isrc, g.dt * snext);
       snext = s_fwd[(size_t)s * (g.nt + 1) + it - 1];
     }
-    if (T.f & kSide)
-      tile_p<TX, true>(T, r, tt0, p, u, w, c1, c2);
-    else
-      tile_p<TX, false>(T, r, tt0, p, u, w, c1, c2);
+    tile_p<TX>(T, r, tt0, p, u, w, c1, c2);
     if (T.f & kAdj) {
       if ((T.f & kRare) && (T.f & kEnds)) zero_cols<TX>(T.ix0, p, 3, NX - 2);
       if (rec.comp == 0) {

@@ -80,7 +80,7 @@ __device__ __forceinline__ void xtile_p(const Tile<TX>& T, const ResPlan& r, flo
 }
 
 // lw from A lp.
-template <int TX, bool SIDE>
+template <int TX>
 __device__ __forceinline__ void xtile_w(const Tile<TX>& T, const ResPlan& r, int tt0, const float (&al)[TX][4],
                                         float (&w)[TX][4], float c1, float c2) {
   const int lane = threadIdx.x & 31;
@@ -91,8 +91,8 @@ __device__ __forceinline__ void xtile_w(const Tile<TX>& T, const ResPlan& r, int
   zrow_get<TX>(r, 1, 2, e6);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
-    float fx = 1.f, z[7];  // A lp at rows -1 .. 5
-    if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).x;
+    const float fx = col_factor<TX>(T, r, tt0, c).x;
+    float z[7];  // A lp at rows -1 .. 5
     z[0] = __shfl_up_sync(0xffffffffu, al[c][3], 1);
     z[5] = __shfl_down_sync(0xffffffffu, al[c][0], 1);
     z[6] = __shfl_down_sync(0xffffffffu, al[c][1], 1);
@@ -103,7 +103,7 @@ __device__ __forceinline__ void xtile_w(const Tile<TX>& T, const ResPlan& r, int
     for (int j = 0; j < 4; ++j) z[1 + j] = al[c][j];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float a = (SIDE ? fminf(fx, fz[j]) : fz[j]) * w[c][j];
+      float a = fminf(fx, fz[j]) * w[c][j];
       a = a - c1 * z[j + 1];
       a = a + c1 * z[j + 2];
       a = a - c2 * z[j];
@@ -113,7 +113,7 @@ __device__ __forceinline__ void xtile_w(const Tile<TX>& T, const ResPlan& r, int
 }
 
 // lu from A lp (x-neighbours in the edge arrays).
-template <int TX, bool SIDE>
+template <int TX>
 __device__ __forceinline__ void xtile_u(const Tile<TX>& T, const ResPlan& r, int tt0, const float (&al)[TX][4],
                                         float (&u)[TX][4], float c1, float c2) {
   float pm1[4], pp1[4], pp2[4], fz[4];
@@ -123,14 +123,13 @@ __device__ __forceinline__ void xtile_u(const Tile<TX>& T, const ResPlan& r, int
   lds4(T.e + kEdge * r.nq + 1, pp2);
 #pragma unroll
   for (int c = 0; c < TX; ++c) {
-    float fx = 1.f;
-    if constexpr (SIDE) fx = col_factor<TX>(T, r, tt0, c).y;
+    const float fx = col_factor<TX>(T, r, tt0, c).y;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float l1 = c >= 1 ? al[c >= 1 ? c - 1 : 0][j] : pm1[j];
       const float r1 = c + 1 < TX ? al[c + 1 < TX ? c + 1 : 0][j] : pp1[j];
       const float r2 = c + 2 < TX ? al[c + 2 < TX ? c + 2 : 0][j] : (c + 1 < TX ? pp1[j] : pp2[j]);
-      float a = (SIDE ? fminf(fx, fz[j]) : fz[j]) * u[c][j];
+      float a = fminf(fx, fz[j]) * u[c][j];
       a = a - c1 * al[c][j];
       a = a + c1 * r1;
       a = a - c2 * l1;
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       lds4(T.rf, fz);
 #pragma unroll
       for (int c = 0; c < TX; ++c) {
-        const float fx = T.f & kSide ? col_factor<TX>(T, r, tt0, c).x : 1.f;
+        const float fx = col_factor<TX>(T, r, tt0, c).x;
 #pragma unroll
         for (int j = 0; j < 4; ++j) p[c][j] = fminf(fx, fz[j]) * p[c][j];
       }
@@ -341,16 +340,10 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (it > it0) prefetch(it - 1);  // the thread's D is read, the other box is free
     __syncthreads();
     // ---- velocity phase
-    if (T.f & kSide)
-      xtile_w<TX, true>(T, r, tt0, al, w, c1, c2);
-    else
-      xtile_w<TX, false>(T, r, tt0, al, w, c1, c2);
+    xtile_w<TX>(T, r, tt0, al, w, c1, c2);
     if (T.f & kRare) xedge_recv<TX>(T, r, gu, dead, al, (unsigned)it, c1, c2);
     __syncwarp();
-    if (T.f & kSide)
-      xtile_u<TX, true>(T, r, tt0, al, u, c1, c2);
-    else
-      xtile_u<TX, false>(T, r, tt0, al, u, c1, c2);
+    xtile_u<TX>(T, r, tt0, al, u, c1, c2);
     if ((T.f & kRare) && (T.f & kEnds)) zero_cols<TX>(T.ix0, u, 2, NX - 2);
 #pragma unroll
     for (int c = 0; c < TX; ++c) {
