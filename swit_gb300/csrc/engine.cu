@@ -1774,7 +1774,7 @@ void multi_release(swit_multi* m) {
 // Instances whose two loops are resident run those, one launch per group of shots, spread over the branch
 // streams: the device schedules a cooperative launch whole, when its blocks fit beside those running, so
 // small problems share it.  6 uneven problems of up to 12 shots 701x251 (gradient): 177.9 ms in waves of the
-// step kernels, 144.1 ms with their resident loops.
+// step kernels, 125.7 ms with their resident loops.
 inline bool multi_resident(const swit_engine* e) { return e->resf && e->resb; }
 
 // Instance table, padded task lists, waves with their block tables and active
@@ -2120,12 +2120,14 @@ void auto_batches(swit_engine* e, int branches) {
 // Resident time loops for FP32 engines on the default kernels and launch
 // shapes, where a split fits the device.  A checkpointed engine runs both loops
 // segment by segment over all shots, so it takes them only together and for
-// segments long enough to pay for loading and storing the state; vx adjoint
+// segments long enough to pay for loading and storing the state (10 shots
+// 801x301, 200 steps: 18.0 against 16.9 ms at 12 steps per segment, 16.0 against
+// 16.5 at 16; 2 shots 182x84, 378 steps: 4.5 against 7.9 at 16); vx adjoint
 // sources change u between the phases, also in the columns a band recomputes,
 // which the resident reverse loop does not do.
 static int res_setup(swit_engine* e, const swit_desc* d) {
   if (d->kernel_variant || e->prec || e->path || d->shots_per_batch || d->graph_branches || d->block_x) return 0;
-  if (e->ckpt_k && e->ckpt_k < 32) return 0;
+  if (e->ckpt_k && e->ckpt_k < 16) return 0;
   ResLoop f, b, x;
   res_choose(e, kResLoopFwd, f);
   if (!e->exact && e->rcomp != 1) res_choose(e, kResLoopBwd, b);

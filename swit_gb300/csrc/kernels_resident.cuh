@@ -819,11 +819,11 @@ __device__ __forceinline__ void list_append(const ResPlan& r, int* cnt, int n, F
 // ---------------------------------------------------------------------------
 // Forward loop, steps it0 .. it1 (fdcore.f90:75-160) of shots shot0 + block / C.
 //
-// Bound by the dependent chain of a step (about 1.6 us: updates, two barriers, the halo) and, with 16 warps
-// on an SM, by issue (2.0 instructions per cycle and SM, 950 per warp and step of which 455 are the
+// Bound by the dependent chain of a step (about 1.4 us: updates, two barriers, the halo) and, with 16 warps
+// on an SM, by issue (about 2 instructions per cycle and SM, 900 per warp and step of which 455 are the
 // stencil's): 512 threads of 128 registers hold as many points as the register file, so a launch takes as
 // many shots as the device holds.  Measured against the vec kernels: 49 shots 481x141, nt 2000, misfit only
-// 56.6 -> 29.3 ms; one shot 101x51, nt 600: 3.05 -> 1.20 ms.
+// 56.4 -> 25.7 ms; one shot 101x51, nt 600: 3.1 -> 0.93 ms.
 template <int TX, int MAXT, bool SAVE>
 __global__ void __launch_bounds__(MAXT, 1)
     k_fwd_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,
@@ -1041,8 +1041,8 @@ __device__ __forceinline__ void side_insert(const Tile<TX>& T, const ResPlan& r,
 //
 // Five 16-value arrays and the rest need more registers than 128: 384 threads of 168 are faster on a full
 // device than 512 of 128, which spill (49 shots 481x141: 3.1 against 4.4 us per step and launch, 13 and 10
-// launches).  Measured against the vec kernels: reverse loop of 49 shots 481x141, nt 1000: 59.8 -> 40.4 ms;
-// of 5 shots 201x101, nt 2000: 22.4 -> 5.7 ms.
+// launches, before later steps).  Measured against the vec kernels: reverse step of 49 shots 481x141
+// 59.8 -> 35.5 us, of 5 shots 201x101 11.2 -> 2.4 us.
 template <int TX, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
     k_bwd_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,

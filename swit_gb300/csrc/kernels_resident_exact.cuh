@@ -204,8 +204,8 @@ __device__ __forceinline__ void xedge_recv(const Tile<TX>& T, const ResPlan& r, 
 // per column, consecutive in a warp.  384 threads of 168 registers, for four 16-value arrays.
 //
 // Bound by the dependent chain of a step, and on a full device by issue.  10 shots 241x121, per step, against
-// the kernels of kernels_exact.cuh: forward keeping D 2.15, reverse 2.63 us, together 18.8 -> 4.8 us (gradient
-// of 1200 steps 22.5 -> 5.7 ms); 20 shots 481x141: 6.2 and 10.1 us.
+// the kernels of kernels_exact.cuh: forward keeping D 1.95, reverse 2.59 us, together 18.8 -> 4.5 us (gradient
+// of 1200 steps 22.5 -> 5.3 ms); 20 shots 481x141: 5.7 and 9.9 us.
 template <int TX, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
     k_xadj_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,

@@ -86,7 +86,7 @@ def test_reverse_matches_oracle(shape, tiles, monkeypatch):
             np.testing.assert_array_equal(a, want[k], err_msg=k)
 
 
-@pytest.mark.parametrize("every", [32, 50, 139, 140])
+@pytest.mark.parametrize("every", [16, 32, 50, 139, 140])
 def test_checkpointed_segments_match_oracle(every, monkeypatch):
     """Segments of a checkpointed run start and end in the fields the loop before left in memory."""
     s, pb = problem()
@@ -105,7 +105,7 @@ def test_checkpointed_segments_match_oracle(every, monkeypatch):
 
 @pytest.mark.parametrize("cols", [4, 8])
 @pytest.mark.parametrize("shape,tiles,every", [(a, t, 0) for a, t in SHAPES if "comp" not in a] +
-                         [(dict(), 2, k) for k in (32, 50, 139, 140)])
+                         [(dict(), 2, k) for k in (16, 50, 139, 140)])
 def test_exact_adjoint_matches_oracle(shape, tiles, every, cols, monkeypatch):
     s, pb = problem(**shape)
     src, rho = s.source(), s.rho(s.vp_true)
@@ -131,7 +131,7 @@ def test_routes():
     s, _ = problem()
     for opts, kernel in ((dict(), "resident"), (dict(kernel="vec"), "vec"), (dict(shots_per_batch=1), "vec"),
                          (dict(precision="fp64"), "vec"), (dict(path="plain"), "vec"), (dict(graph_branches=2), "vec"),
-                         (dict(block_x=8), "vec"), (dict(checkpoint_every=31), "vec"),
+                         (dict(block_x=8), "vec"), (dict(checkpoint_every=15), "vec"),
                          (dict(receiver_component="vx"), "vec"), (dict(adjoint="exact"), "resident"),
                          (dict(adjoint="exact", receiver_component="vz"), "vec")):
         with Engine(**s.engine_args(), **opts) as e:
