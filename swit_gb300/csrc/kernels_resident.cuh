@@ -820,7 +820,7 @@ __device__ __forceinline__ void list_append(const ResPlan& r, int* cnt, int n, F
 // Forward loop, steps it0 .. it1 (fdcore.f90:75-160) of shots shot0 + block / C.
 //
 // Bound by the dependent chain of a step (about 1.4 us: updates, two barriers, the halo) and, with 16 warps
-// on an SM, by issue (about 2 instructions per cycle and SM, 900 per warp and step of which 455 are the
+// on an SM, by issue (2.2 instructions per cycle and SM, 940 per warp and step of which 455 are the
 // stencil's): 512 threads of 128 registers hold as many points as the register file, so a launch takes as
 // many shots as the device holds.  Measured against the vec kernels: 49 shots 481x141, nt 2000, misfit only
 // 56.4 -> 25.7 ms; one shot 101x51, nt 600: 3.1 -> 0.93 ms.
