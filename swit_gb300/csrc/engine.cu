@@ -1026,14 +1026,21 @@ int residual_l2(swit_engine* e, const float* obs, int on_device, cudaStream_t st
   return 0;
 }
 
+// End of a call that waits for its results: synchronises, and reports a halo wait of the resident loops that
+// gave up.
+int host_end(swit_engine* e, cudaStream_t st) {
+  int err = 0;
+  if (e->d_halo) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (!err) return 0;
+  return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
+}
+
 // Sum of the per-trace misfits on the host (waits for the stream).
 int misfit_sum(swit_engine* e, cudaStream_t st, double* misfit) {
   std::vector<double> mt((size_t)e->ns * e->ngmax);
-  int err = 0;
   CK(cudaMemcpyAsync(mt.data(), e->d_mtrace, mt.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (e->resf) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (err) return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
+  if (const int rc = host_end(e, st)) return rc;
   double acc = 0.0;
   for (double v : mt) acc += v;
   *misfit = acc;
@@ -1191,8 +1198,7 @@ int export_impl(swit_engine* e, void* boundary, void* pend, void* uend, void* we
     });
     if (rc) return rc;
   }
-  if (!on_device) CK(cudaStreamSynchronize(st));
-  return 0;
+  return on_device ? 0 : host_end(e, st);
 }
 
 // Per-launch timing of the stencil kernels with CUDA events.
@@ -2485,15 +2491,6 @@ int swit_create(const swit_desc* d, swit_engine** out) {
   return 0;
 }
 
-// End of a call with host buffers: waits for the stream; the resident loops report a wait that gave up.
-static int host_end(swit_engine* e, cudaStream_t st) {
-  int err = 0;
-  if (e->resf) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (err) return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
-  return 0;
-}
-
 int swit_set_model(swit_engine* e, const float* vp, const float* rho, int on_device, void* stream) {
   if (!e || !vp || !rho) return fail(SWIT_E_ARG, "null argument");
   cudaStream_t st = (cudaStream_t)stream;
@@ -2543,8 +2540,7 @@ int swit_gradient_l2(swit_engine* e, const float* src, const float* obs, void* g
   int rc = e->prec ? gradient_impl<double>(e, src, obs, grad, illum_fw, illum_bk, seis, misfit, on_device, st)
                    : gradient_impl<float>(e, src, obs, grad, illum_fw, illum_bk, seis, misfit, on_device, st);
   if (rc) return rc;
-  if (!on_device) CK(cudaStreamSynchronize(st));
-  return 0;
+  return on_device ? 0 : host_end(e, st);
 }
 
 int swit_backward_exact(swit_engine* e, const float* adj, void* grad, void* src_grad, int on_device, void* stream) {
@@ -2556,8 +2552,7 @@ int swit_backward_exact(swit_engine* e, const float* adj, void* grad, void* src_
   int rc = e->prec ? exact_impl<double>(e, adj, grad, src_grad, on_device, st)
                    : exact_impl<float>(e, adj, grad, src_grad, on_device, st);
   if (rc) return rc;
-  if (!on_device) CK(cudaStreamSynchronize(st));
-  return 0;
+  return on_device ? 0 : host_end(e, st);
 }
 
 int swit_export_snapshot(swit_engine* e, void* boundary, void* p_end, void* u_end, void* w_end, int on_device,
@@ -2736,10 +2731,12 @@ int swit_multi_gradient_l2(swit_multi* m, const float* const* src, const float* 
                              illum_bk ? illum_bk[i] : nullptr, on_device, st);
     if (rc) return rc;
   }
-  if (misfit)
-    for (int i = 0; i < n; ++i)
-      if ((rc = misfit_sum(m->eng[i], st, &misfit[i]))) return rc;
-  return 0;
+  int first = 0;
+  for (int i = 0; i < n && (misfit || !on_device); ++i) {
+    rc = misfit ? misfit_sum(m->eng[i], st, &misfit[i]) : host_end(m->eng[i], st);
+    if (rc && !first) first = rc;
+  }
+  return first;
 }
 
 int swit_multi_misfit_l2(swit_multi* m, const float* const* src, const float* const* obs, const int32_t* active,
@@ -2762,11 +2759,12 @@ int swit_multi_misfit_l2(swit_multi* m, const float* const* src, const float* co
   if (rc) return rc;
   for (int i = 0; i < n; ++i)
     if (on[i] && (rc = residual_l2<float>(m->eng[i], obs[i], on_device, st))) return rc;
+  int first = 0;
   for (int i = 0; i < n; ++i) {
     misfit[i] = 0.0;
-    if (on[i] && (rc = misfit_sum(m->eng[i], st, &misfit[i]))) return rc;
+    if (on[i] && (rc = misfit_sum(m->eng[i], st, &misfit[i])) && !first) first = rc;
   }
-  return 0;
+  return first;
 }
 
 int swit_multi_destroy(swit_multi* m) {
