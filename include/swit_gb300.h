@@ -269,8 +269,9 @@ int swit_backward_exact(swit_engine* e, const float* adj, void* grad, void* src_
  * SWIT_E_TIMEOUT once for such an event, then clears it.  With the resident
  * loops, calls with host buffers and calls that return a misfit report the event
  * themselves (the call that fails, or the first of them after device-buffer calls
- * that did).  No counterpart in the reference, whose CPU loops have no
- * asynchronous copies. */
+ * that did); a report leaves later calls unaffected, but the saved forward run
+ * is then no longer there for swit_backward.  No counterpart in the reference,
+ * whose CPU loops have no asynchronous copies. */
 int swit_check(swit_engine* e, void* stream);
 
 /* The Waveform misfit of swit_gradient_l2 alone: a forward run without strips,

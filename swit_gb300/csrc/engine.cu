@@ -142,7 +142,8 @@ struct swit_engine {
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
   // resident time loops (kernels_resident.cuh), where the split fits the device; else the variant's kernels
   ResLoop *resf = nullptr, *resb = nullptr, *resx = nullptr;  // forward, reverse, exact adjoint's reverse
-  uint4* d_halo = nullptr;
+  uint4* d_halo = nullptr;  // packet 0: a launch's stop word; then its halo packets
+  int wait_err = 0;         // error word that a call has reported and swit_check has not
 };
 
 namespace {
@@ -1027,12 +1028,16 @@ int residual_l2(swit_engine* e, const float* obs, int on_device, cudaStream_t st
 }
 
 // End of a call that waits for its results: synchronises, and reports a halo wait of the resident loops that
-// gave up.
+// gave up since the last report.  The word is cleared, so that later calls are judged by their own waits; a saved
+// forward run is not used any more (it may be what went wrong); swit_check still reports the word once.
 int host_end(swit_engine* e, cudaStream_t st) {
   int err = 0;
   if (e->d_halo) CK(cudaMemcpyAsync(&err, e->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (!err) return 0;
+  e->wait_err = err;
+  e->fwd_ready = false;
+  CK(cudaMemsetAsync(e->d_err, 0, sizeof(int), st));
   return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting (error word %d); results are invalid", err);
 }
 
@@ -2141,13 +2146,13 @@ static int res_setup(swit_engine* e, const swit_desc* d) {
   if (e->ckpt_k && !e->exact && !(f.ok && b.ok)) return 0;
   const size_t n = std::max(std::max(res_halo_packets(f), res_halo_packets(b)), res_halo_packets(x));
   if (!n) return 0;
-  if (int rc = dalloc(e, &e->d_halo, n)) return rc;
+  if (int rc = dalloc(e, &e->d_halo, n + 1)) return rc;
   unsigned wait = kResWaitLimit;
   if (const char* v = std::getenv("SWIT_RES_WAIT_POLLS")) {  // a shorter wait, e.g. to test the timeout path
     const long long w = std::atoll(v);
     if (w >= 0 && w < (long long)kResWaitLimit) wait = (unsigned)w;
   }
-  f.r.halo = b.r.halo = x.r.halo = e->d_halo;
+  f.r.halo = b.r.halo = x.r.halo = e->d_halo + 1;
   f.r.err = b.r.err = x.r.err = e->d_err;
   f.r.wait = b.r.wait = x.r.wait = wait;
   if (f.ok) e->resf = new ResLoop(f);
@@ -2645,8 +2650,11 @@ int swit_check(swit_engine* e, void* stream) {
   CK(cudaStreamSynchronize((cudaStream_t)stream));
   int w = 0;
   CK(cudaMemcpy(&w, e->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  if (w) CK(cudaMemset(e->d_err, 0, sizeof(int)));
+  if (w && e->d_halo) e->fwd_ready = false;
+  if (!w) w = e->wait_err;
+  e->wait_err = 0;
   if (w) {
-    CK(cudaMemset(e->d_err, 0, sizeof(int)));
     return fail(SWIT_E_TIMEOUT, "a kernel gave up waiting for its copies or a neighbour's halo (error word %d); results are invalid", w);
   }
   return 0;
@@ -2731,6 +2739,7 @@ int swit_multi_gradient_l2(swit_multi* m, const float* const* src, const float* 
                              illum_bk ? illum_bk[i] : nullptr, on_device, st);
     if (rc) return rc;
   }
+  // every instance's wait is looked at, so that none is left for a later call to report
   int first = 0;
   for (int i = 0; i < n && (misfit || !on_device); ++i) {
     rc = misfit ? misfit_sum(m->eng[i], st, &misfit[i]) : host_end(m->eng[i], st);

@@ -26,7 +26,9 @@
 // same values as in the neighbour.  A packet slot is reused two steps later; the
 // neighbour can only be that far ahead after every thread of this block has left
 // the phase that reads it.  Every poll is bounded; a thread that gives up
-// records it in the engine's error word and does not wait again.
+// records it in the engine's error word, which stays until a call reports it, and
+// in the launch's stop word, at which the other threads soon give up too; it does
+// not wait again.
 //
 // Damping.  The reference's profile is damp(max(iX, iZ)) with iX, iZ the cell
 // numbers from the inner edges and damp non-decreasing, and rounding is
@@ -77,8 +79,8 @@ struct ResPlan {
   int nside;     // side arrays a band may hold: 6, or the 3 of one side
   float negz;    // -0 (see f2)
   unsigned wait; // polls before a halo wait gives up
-  uint4* halo;   // packets: [block][role][side][parity][packet][row tile]
-  int* err;
+  uint4* halo;   // packets: [block][role][side][parity][packet][row tile]; the stop word lies one packet before
+  int* err;      // the engine's error word
   // A thread's data lies together at an odd stride of float4: addresses are a base and a constant, and the
   // 16-byte accesses of a warp are free of bank conflicts.
   int oC;        // coefficients of a thread: p update [TX], u, w updates [TX]; stride 2 TX + 1
@@ -225,7 +227,9 @@ __device__ __forceinline__ void halo_wait(const uint4* p, unsigned tag, const Re
   for (unsigned n = 0;; ++n) {
     halo_issue(p, r.nq, h);
     if (halo_here(h, tag) || dead) return;
-    if (n >= r.wait || ((n & 255u) == 255u && *(volatile int*)r.err != 0)) {
+    int* stop = reinterpret_cast<int*>(r.halo - 1);
+    if (n >= r.wait || ((n & 255u) == 255u && *(volatile int*)stop != 0)) {
+      atomicExch(stop, 1);
       atomicCAS(r.err, 0, kResErr);
       dead = true;
     }

@@ -88,3 +88,25 @@ def test_multi_engine_without_misfits_reports_every_instance(monkeypatch):
             with timeout():
                 e.check()
             e.check()
+
+
+def test_a_reported_wait_leaves_later_calls_alone(monkeypatch):
+    """After the report the forward run counts as not made, and calls whose own waits are in order
+    succeed without a swit_check between."""
+    s, pb, src, rho = problem()
+    ref = O.forward(pb, s.vp_true, rho, src, store=True)
+    adj = (ref["seis"] * 0.5).astype(np.float32)
+    want = O.adjoint(pb, s.vp_true, rho, src, adj, ref)
+    bands(monkeypatch, 1, 100)
+    with Engine(**s.engine_args()) as e:
+        e.set_model(s.vp_true, rho)
+        with timeout():
+            e.forward(src, save_boundary=True)
+        with pytest.raises(SwitError, match="SWIT_E_STATE"):
+            e.backward(adj)
+        e.import_snapshot(src, *[ref[k] for k in ("boundary", "p_end", "u_end", "w_end")])
+        for a, k in zip(e.backward(adj), ("g", "fw", "bk")):
+            np.testing.assert_array_equal(a, want[k], err_msg=k)
+        with timeout():
+            e.check()  # still reports the forward, once
+        e.check()
