@@ -113,9 +113,9 @@ typedef struct swit_desc {
   int32_t graph_branches;   /* batched path: the shot batches' step chains form
                                this many concurrent branches of the captured
                                graphs (batch b on branch b mod graph_branches);
-                               0 = automatic (with automatic shots_per_batch as
-                               many as shots whose state fits in L2, at most 3;
-                               else 2), at most 4                               */
+                               0 = automatic (with automatic shots_per_batch 3,
+                               or fewer where the FP32 vec kernels' shots in
+                               flight would not fit the L2; else 2), at most 4  */
   int32_t adjoint_mode;     /* 0 = fd2dmpi's adjoint (boundary strips, reverse
                                reconstruction, continuous-adjoint imaging:
                                swit_backward); 1 = exact discrete adjoint of the
@@ -249,6 +249,14 @@ int swit_forward_shot_static(int32_t nx, int32_t nz, int32_t npml, int32_t nt, f
 int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_batch, int32_t* block_x,
                int32_t* kernels_per_forward, int32_t* kernels_per_backward, int32_t* kernel_variant,
                int32_t* graph_branches);
+
+/* What one time loop runs: loop 0 = forward without strips, 1 = forward that
+ * saves them (or the exact adjoint's divergence; with checkpoints the forward of
+ * a segment), 2 = reverse.  kernel_variant as swit_query's; shots per launch;
+ * threads per block of a resident loop (0 otherwise); concurrent graph branches
+ * (1 for a resident loop).  Any output may be NULL. */
+int swit_query_loop(const swit_engine* e, int32_t loop, int32_t* kernel_variant, int32_t* shots, int32_t* threads,
+                    int32_t* branches);
 
 /* Exact discrete adjoint (engines created with adjoint_mode = 1) after a
  * swit_forward with save_boundary = 1: the transpose of the forward map applied

@@ -15,7 +15,8 @@ ERRORS = {-1: "SWIT_E_ARG", -2: "SWIT_E_GEOM", -3: "SWIT_E_CFL", -4: "SWIT_E_MOD
 
 # every symbol include/swit_gb300.h declares
 EXPORTS = ("swit_create", "swit_set_model", "swit_forward", "swit_backward", "swit_gradient_l2",
-           "swit_export_snapshot", "swit_import_snapshot", "swit_profile_kernels", "swit_backward_exact", "swit_query", "swit_destroy", "swit_last_error", "swit_damp_profile",
+           "swit_export_snapshot", "swit_import_snapshot", "swit_profile_kernels", "swit_backward_exact", "swit_query", "swit_query_loop",
+           "swit_destroy", "swit_last_error", "swit_damp_profile",
            "swit_forward_shot_static", "swit_check", "swit_misfit_l2", "swit_multi_create", "swit_multi_engine",
            "swit_multi_gradient_l2", "swit_multi_misfit_l2", "swit_multi_destroy", "swit_l2_bandwidth")
 
@@ -64,6 +65,7 @@ def load(build_if_missing: bool = True):
         "swit_backward_exact": ([vp, vp, vp, vp, C.c_int32, vp], i),
         "swit_query": ([vp, C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                         C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32), C.POINTER(C.c_int32)], i),
+        "swit_query_loop": ([vp, C.c_int32] + [C.POINTER(C.c_int32)] * 4, i),
         "swit_destroy": ([vp], i),
         "swit_check": ([vp, vp], i),
         "swit_misfit_l2": ([vp, vp, vp, C.POINTER(C.c_double), C.c_int32, vp], i),

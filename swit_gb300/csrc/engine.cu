@@ -66,6 +66,7 @@ struct swit_engine {
   int nx, nz, L, nt, NX, NZ, LD, LDI, fs, fs_flag, ns, ngmax, SL, prec, path;
   float dx32, dt32;
   int batch, bx;
+  int fbatch = 0;  // shots per launch of the forward loop's step kernels (batch: the reverse loop's)
   int variant;  // 1 = split, 2 = walk (one kernel per step, ping-pong), 3 = vec (split, 4 rows per thread),
                 // 4 = cluster (one persistent cluster per shot, wavefields in distributed shared memory),
                 // 5 = hybrid (cluster forward, vec reverse loop), 6 = band (vec bodies on bands of
@@ -128,7 +129,7 @@ struct swit_engine {
   cudaStream_t cpy = nullptr;
   cudaEvent_t ev_in = nullptr, ev_cpy = nullptr;
   float* d_src_in = nullptr;  // source staging (ns x nt floats), apart from d_in
-  int branches = 2;  // graph branches in use (swit_desc.graph_branches)
+  int branches = 2, fbranches = 2;  // graph branches in use, reverse and forward (swit_desc.graph_branches)
   // captured loops, each a sequence of graphs of at most kGraphNodes nodes (capture_chunked)
   std::vector<cudaGraphExec_t> gfwd[2];
   std::vector<cudaGraphExec_t> gbwd;
@@ -490,7 +491,7 @@ void launch_backward_steps(swit_engine* e, int shot0, int nb, cudaStream_t st, i
 
 // Shots per forward launch: the hybrid variant runs every shot in one cluster
 // launch (the hardware schedules the clusters); the others use the batch.
-inline int fwd_batch(const swit_engine* e) { return e->variant == 5 ? e->ns : e->batch; }
+inline int fwd_batch(const swit_engine* e) { return e->variant == 5 ? e->ns : e->fbatch; }
 
 // Checkpointed recomputation.  Segment m (m = 0 .. ckpt_m-1, ckpt_m =
 // ceil(nt/k)) is the forward steps [max(2, m k + 1), min(nt, (m+1) k)]; the
@@ -613,16 +614,16 @@ void exact_reverse(swit_engine* e, int s0, int nb, cudaStream_t st, bool res = f
 // per branch (auto_batches): at 481x141, 127.6 shot-gradients/s with three
 // branches of 9-shot batches, 126.0 with two of 13, 105.3 with 13-shot batches
 // on three branches (one branch runs two batches) and 101.6 with one chain.
-inline cudaStream_t capture_stream(swit_engine* e, int b, cudaStream_t origin) {
-  const int k = b % e->branches;
+inline cudaStream_t capture_stream(swit_engine* e, int branches, int b, cudaStream_t origin) {
+  const int k = b % branches;
   return k ? e->capx[k - 1] : origin;
 }
-inline void capture_fork(swit_engine* e, cudaStream_t origin) {
+inline void capture_fork(swit_engine* e, int branches, cudaStream_t origin) {
   cudaEventRecord(e->ev_fork, origin);
-  for (int i = 0; i < e->branches - 1; ++i) cudaStreamWaitEvent(e->capx[i], e->ev_fork, 0);
+  for (int i = 0; i < branches - 1; ++i) cudaStreamWaitEvent(e->capx[i], e->ev_fork, 0);
 }
-inline void capture_join(swit_engine* e, cudaStream_t origin) {
-  for (int i = 0; i < e->branches - 1; ++i) {
+inline void capture_join(swit_engine* e, int branches, cudaStream_t origin) {
+  for (int i = 0; i < branches - 1; ++i) {
     cudaEventRecord(e->ev_join[i], e->capx[i]);
     cudaStreamWaitEvent(origin, e->ev_join[i], 0);
   }
@@ -652,21 +653,21 @@ inline int launch_graphs(const std::vector<cudaGraphExec_t>& ex, cudaStream_t st
 
 // Captures batches 0 .. nbatch-1 (issue(b, stream) launches batch b's work on
 // the given capture stream) into ex: consecutive chunks of batches, each chunk
-// one graph with the batches on concurrent branches.  ex is left empty on error.
+// one graph with the batches on `branches` concurrent branches.  ex is left empty on error.
 template <class F>
-int capture_chunked(swit_engine* e, std::vector<cudaGraphExec_t>& ex, int nbatch, size_t nodes_per_batch,
+int capture_chunked(swit_engine* e, std::vector<cudaGraphExec_t>& ex, int branches, int nbatch, size_t nodes_per_batch,
                     const char* what, F&& issue) {
   int chunk = (int)std::max<size_t>(1, e->graph_nodes / std::max<size_t>(1, nodes_per_batch));
-  if (chunk >= e->branches) chunk -= chunk % e->branches;
+  if (chunk >= branches) chunk -= chunk % branches;
   for (int b0 = 0; b0 < nbatch; b0 += chunk) {
     cudaError_t rc = cudaStreamBeginCapture(e->cap, cudaStreamCaptureModeThreadLocal);
     if (rc != cudaSuccess) {
       destroy_graphs(ex);
       return fail(SWIT_E_CUDA, "%s graph capture: %s", what, cudaGetErrorString(rc));
     }
-    capture_fork(e, e->cap);
-    for (int b = b0; b < std::min(nbatch, b0 + chunk); ++b) issue(b, capture_stream(e, b - b0, e->cap));
-    capture_join(e, e->cap);
+    capture_fork(e, branches, e->cap);
+    for (int b = b0; b < std::min(nbatch, b0 + chunk); ++b) issue(b, capture_stream(e, branches, b - b0, e->cap));
+    capture_join(e, branches, e->cap);
     cudaGraph_t graph = nullptr;
     rc = cudaStreamEndCapture(e->cap, &graph);
     if (rc != cudaSuccess) {
@@ -694,7 +695,7 @@ inline bool caller_capturing(cudaStream_t st) {
 }
 
 template <class F>
-int issue_into_capture(swit_engine* e, cudaStream_t st, int nbatch, F&& issue) {
+int issue_into_capture(swit_engine* e, cudaStream_t st, int branches, int nbatch, F&& issue) {
   // the caller's graph gets every node of the loop: keep it under the same bound
   // as the engine's own graphs
   const size_t nodes = (size_t)nbatch * loop_nodes(e);
@@ -703,9 +704,9 @@ int issue_into_capture(swit_engine* e, cudaStream_t st, int nbatch, F&& issue) {
                 "capturing this loop into the caller's graph would add about %zu kernel nodes, above the %zu-node "
                 "bound of one graph; run it uncaptured (the engine then splits it into bounded graphs itself)",
                 nodes, e->graph_nodes);
-  capture_fork(e, st);
-  for (int b = 0; b < nbatch; ++b) issue(b, capture_stream(e, b, st));
-  capture_join(e, st);
+  capture_fork(e, branches, st);
+  for (int b = 0; b < nbatch; ++b) issue(b, capture_stream(e, branches, b, st));
+  capture_join(e, branches, st);
   CK(cudaGetLastError());
   return 0;
 }
@@ -741,9 +742,9 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
     else
       launch_forward_steps<R>(e, store, s0, nb, cs);
   };
-  if (caller_capturing(st)) return issue_into_capture(e, st, nbatch, issue);
+  if (caller_capturing(st)) return issue_into_capture(e, st, e->fbranches, nbatch, issue);
   if (ex.empty()) {
-    int rc = capture_chunked(e, ex, nbatch, loop_nodes(e), "forward", issue);
+    int rc = capture_chunked(e, ex, e->fbranches, nbatch, loop_nodes(e), "forward", issue);
     if (rc) return rc;
   }
   return launch_graphs(ex, st);
@@ -777,9 +778,9 @@ int run_backward_loop(swit_engine* e, cudaStream_t st) {
     else
       launch_backward_steps<R>(e, s0, nb, cs);
   };
-  if (caller_capturing(st)) return issue_into_capture(e, st, nbatch, issue);
+  if (caller_capturing(st)) return issue_into_capture(e, st, e->branches, nbatch, issue);
   if (e->gbwd.empty()) {
-    int rc = capture_chunked(e, e->gbwd, nbatch, loop_nodes(e), "backward", issue);
+    int rc = capture_chunked(e, e->gbwd, e->branches, nbatch, loop_nodes(e), "backward", issue);
     if (rc) return rc;
   }
   return launch_graphs(e->gbwd, st);
@@ -888,9 +889,9 @@ int run_exact_loop(swit_engine* e, cudaStream_t st) {
   auto issue = [&](int b, cudaStream_t cs) {
     exact_reverse<R>(e, b * e->batch, std::min(e->batch, e->ns - b * e->batch), cs);
   };
-  if (caller_capturing(st)) return issue_into_capture(e, st, nbatch, issue);
+  if (caller_capturing(st)) return issue_into_capture(e, st, e->branches, nbatch, issue);
   if (e->gxb.empty()) {
-    int rc = capture_chunked(e, e->gxb, nbatch, loop_nodes(e), "exact adjoint", issue);
+    int rc = capture_chunked(e, e->gxb, e->branches, nbatch, loop_nodes(e), "exact adjoint", issue);
     if (rc) return rc;
   }
   return launch_graphs(e->gxb, st);
@@ -1219,13 +1220,13 @@ int export_impl(swit_engine* e, void* boundary, void* pend, void* uend, void* we
 template <class R>
 int profile_vec_graphs(swit_engine* e, int32_t launches[4], double mean_ms[4], cudaStream_t st) {
   Grid<R> g = make_grid<R>(e);
-  const int B = e->batch, nbatch = (e->ns + B - 1) / B;
   const int S = std::min(e->nt - 1, 256);
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   CK(cudaEventCreate(&t0));
   CK(cudaEventCreate(&t1));
   int rc = 0;
   for (int k = 0; k < 4 && !rc; ++k) {
+    const int B = k < 2 ? fwd_batch(e) : e->batch, nbatch = (e->ns + B - 1) / B, br = k < 2 ? e->fbranches : e->branches;
     auto issue = [&](int b, cudaStream_t cs) {
       const int s0 = b * B, nb = std::min(B, e->ns - s0);
       for (int i = 0; i < S; ++i) {
@@ -1250,7 +1251,7 @@ int profile_vec_graphs(swit_engine* e, int32_t launches[4], double mean_ms[4], c
     std::vector<cudaGraphExec_t> ex;
     const size_t saved = e->graph_nodes;
     e->graph_nodes = (size_t)(nbatch + 1) * S;  // one graph per kernel (all batches in one chunk)
-    rc = capture_chunked(e, ex, nbatch, (size_t)S, "profile", issue);
+    rc = capture_chunked(e, ex, br, nbatch, (size_t)S, "profile", issue);
     e->graph_nodes = saved;
     if (rc) break;
     float ms = 0.f;
@@ -2094,7 +2095,7 @@ extern "C" {
 
 const char* swit_last_error(void) { return g_err.c_str(); }
 
-// Automatic shots per launch and graph branches of the vec kernels.  The
+// Automatic shots per launch and graph branches of the vec and walk kernels.  The
 // reverse loop touches per shot 3 wavefields on the PML grid and 6 interior
 // arrays; the step kernels are fastest when the shots of the branches in flight
 // keep that state in L2 (about 0.7 of it, the rest holding strips, traces and
@@ -2102,10 +2103,17 @@ const char* swit_last_error(void) { return g_err.c_str(); }
 // 0.7 L2 / state, branches br (3 unless given), batches k = br * ceil(ns / T)
 // (a multiple of br, so the branches get the same number of launches) and
 // ceil(ns / k) shots per batch.  At 481x141 (npml 40) on GB300: 28 shots in
-// flight, 6 batches of 9 on 3 branches.  Where fewer shots fit, fewer branches
-// run: their state would push each other's out of L2 (reverse step of 3 shots
-// 2001x601: 60.9 us on 3 branches, 53.7 on 2, 58.8 on 1; of 2 shots 3001x801:
-// 85.1 on 2, 81.5 on 1).
+// flight, 6 batches of 9 on 3 branches.
+//
+// Where fewer shots fit, the branches push each other's state out of L2, and the
+// FP32 vec kernels of fd2dmpi's adjoint run fewer, forward and reverse each by
+// the state it touches (us per step on 3, 2 and 1 branches):
+//   reverse, below 2.5 shots: 9 shots 1460x716 152.0, 123.2, 141.9; below 1.5: 7 shots 1884x896 192.6, 188.4,
+//   159.6; a state beyond L2 by itself (below 0.9) has nothing to lose: 3 shots 1915x2337 215.8, 219.4, 227.0;
+//   forward (the 3 wavefields), below 4.5 shots: 7 shots 1884x896 69.5, 61.8, 73.2, above: 9 shots 1460x716
+//   50.0, 55.9, 61.8; below 3: 3 shots 1737x2249 74.0, 68.8, 57.4.
+// FP64, walk and exact-adjoint engines keep 3 at every size: 3 shots 1700x800 FP64 481, 490, 508 reverse and
+// 217, 223, 234 forward; walk 86, 116, 148 and 45, 63, 86.
 void auto_batches(swit_engine* e, int branches) {
   int dev = 0, l2 = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess ||
@@ -2113,19 +2121,31 @@ void auto_batches(swit_engine* e, int branches) {
     l2 = 64 << 20;
   // reverse-loop state per shot: adjoint fields on the PML grid, reconstruction
   // fields and imaging sums on the interior; the walk kernels keep two sets
-  const double state = e->variant == 2 ? (6.0 * e->NX * e->NZ + 9.0 * e->nx * e->nz) * e->esz
-                                       : (3.0 * e->NX * e->NZ + 6.0 * e->nx * e->nz) * e->esz;
+  const double fields = 3.0 * e->NX * e->NZ * e->esz;
+  const double state = e->variant == 2 ? 2 * fields + 9.0 * e->nx * e->nz * e->esz : fields + 6.0 * e->nx * e->nz * e->esz;
   const double fit = 0.7 * l2 / state;
   const int inflight = std::max(1, (int)fit);
-  const int br = std::max(1, std::min(branches ? branches : std::min(3, (int)(fit + 0.5)), e->ns));
-  const int per_branch = std::max(1, inflight / br);
-  const int rounds = (e->ns + br * per_branch - 1) / (br * per_branch);
-  // and at most about 1 M kernel nodes per captured loop (grids whose state
-  // does not fit the L2 would otherwise run one shot per launch)
-  const int kmax = std::max(br, (int)(((size_t)1 << 20) / (2 * (size_t)(e->nt - 1))) / br * br);
-  const int k = std::min(std::min(e->ns, br * rounds), kmax);
-  e->batch = (e->ns + k - 1) / k;
-  e->branches = br;
+  auto rounds = [&](int br) {  // launches of a branch per step
+    const int per = br * std::max(1, inflight / br);
+    return (e->ns + per - 1) / per;
+  };
+  auto batch = [&](int br) {
+    // at most about 1 M kernel nodes per captured loop (grids whose state
+    // does not fit the L2 would otherwise run one shot per launch)
+    const int kmax = std::max(br, (int)(((size_t)1 << 20) / (2 * (size_t)(e->nt - 1))) / br * br);
+    const int k = std::min(std::min(e->ns, br * rounds(br)), kmax);
+    return (e->ns + k - 1) / k;
+  };
+  e->branches = e->fbranches = std::min(branches ? branches : 3, e->ns);
+  if (!branches && e->variant == 3 && !e->prec && !e->exact) {
+    if (fit >= 0.9) e->branches = std::min(e->branches, std::max(1, (int)(fit + 0.5)));
+    const double ffit = 0.7 * l2 / fields;
+    e->fbranches = std::min(e->fbranches, ffit >= 4.5 ? 3 : (ffit >= 3.0 ? 2 : 1));
+    // no more rounds on the reverse loop's fewer branches (4 shots 1131x1141: 26.7 on 3, 24.3 on 2)
+    if (e->branches < e->fbranches && rounds(e->branches) == rounds(e->fbranches)) e->fbranches = e->branches;
+  }
+  e->batch = batch(e->branches);
+  e->fbatch = batch(e->fbranches);
 }
 
 // Resident time loops for FP32 engines on the default kernels and launch
@@ -2268,7 +2288,8 @@ int swit_create(const swit_desc* d, swit_engine** out) {
     return fail(SWIT_E_ARG, "graph_branches must be 0 (automatic) or 1..%d (got %d)", kCapStreamsMax,
                 d->graph_branches);
   }
-  e->branches = d->graph_branches ? d->graph_branches : 2;
+  e->branches = e->fbranches = d->graph_branches ? d->graph_branches : 2;
+  e->fbatch = e->batch;
   e->graph_nodes = kGraphNodes;
   e->band_wait = kBandWaitLimit;
   if (const char* bw = std::getenv("SWIT_BAND_WAIT_POLLS")) {  // a shorter wait, e.g. to test the timeout path
@@ -2642,6 +2663,21 @@ int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_b
   if (kernels_per_forward) *kernels_per_forward = e->launches_fwd;
   if (kernels_per_backward) *kernels_per_backward = e->launches_bwd;
   if (kernel_variant) *kernel_variant = e->resf && (e->resb || e->resx) ? 7 : e->variant;
+  return 0;
+}
+
+int swit_query_loop(const swit_engine* e, int32_t loop, int32_t* kernel_variant, int32_t* shots, int32_t* threads,
+                    int32_t* branches) {
+  if (!e) return fail(SWIT_E_ARG, "null argument");
+  if (loop < 0 || loop > 2) return fail(SWIT_E_ARG, "loop must be 0 (forward), 1 (saving forward) or 2 (reverse) (got %d)", loop);
+  const ResLoop* l = loop == 2 ? (e->exact ? e->resx : e->resb) : e->resf;
+  if (loop == 1 && e->exact && !e->ckpt_k && !e->resx) l = nullptr;
+  const int batch = e->path == 1 ? 1 : (loop == 2 ? e->batch : fwd_batch(e));
+  const int br = e->path == 1 ? 1 : std::min(loop == 2 ? e->branches : e->fbranches, (e->ns + batch - 1) / batch);
+  if (kernel_variant) *kernel_variant = l ? 7 : e->variant;
+  if (shots) *shots = l ? l->shots : batch;
+  if (threads) *threads = l ? l->r.nA + l->r.nR : 0;
+  if (branches) *branches = l ? 1 : br;
   return 0;
 }
 

@@ -13,6 +13,9 @@ import numpy as np
 from . import _lib
 
 
+_KERNELS = {1: "split", 2: "walk", 3: "vec", 4: "cluster", 5: "hybrid", 6: "band", 7: "resident"}
+
+
 def _is_torch(a):
     return type(a).__module__.split(".")[0] == "torch"
 
@@ -234,6 +237,14 @@ class Engine:
             names = ("fwd_loop", None, "bwd_uw", "bwd_p")
         return {k: dict(launches=int(n[i]), mean_ms=float(ms[i])) for i, k in enumerate(names) if k}
 
+    def query_loop(self, loop):
+        """What a time loop runs, loop "forward", "saving" (forward with strips) or "reverse": dict(kernel, shots
+        per launch, threads per block of a resident loop or 0, branches) (swit_query_loop)."""
+        v = [C.c_int32() for _ in range(4)]
+        _lib.check(self._lib.swit_query_loop(self._h, ("forward", "saving", "reverse").index(loop),
+                                             *[C.byref(x) for x in v]))
+        return dict(kernel=_KERNELS.get(v[0].value, "?"), shots=v[1].value, threads=v[2].value, branches=v[3].value)
+
     def query(self):
         by = C.c_int64()
         sb, bx, kf, kb, kv, br = C.c_int32(), C.c_int32(), C.c_int32(), C.c_int32(), C.c_int32(), C.c_int32()
@@ -241,8 +252,7 @@ class Engine:
                                         C.byref(kv), C.byref(br)))
         return dict(device_bytes=by.value, shots_per_batch=sb.value, block_x=bx.value, graph_branches=br.value,
                     kernels_per_forward=kf.value,
-                    kernels_per_backward=kb.value, kernel={1: "split", 2: "walk", 3: "vec", 4: "cluster", 5: "hybrid", 6: "band",
-                            7: "resident"}.get(kv.value, "?"))
+                    kernels_per_backward=kb.value, kernel=_KERNELS.get(kv.value, "?"))
 
     def check(self):
         """Waits for torch's current stream and raises SwitError if a kernel gave
