@@ -208,7 +208,7 @@ inline const ResInst& res_inst(ResKind kind, const ResLoop& l) {
 
 // Launch configuration of `shots` shots; the packets' tags and the stop word before them start from zero.
 inline cudaLaunchConfig_t res_config(const ResLoop& l, int shots, cudaStream_t st, cudaLaunchAttribute* at) {
-  cudaMemsetAsync(l.r.halo - 1, 0, (1 + (size_t)shots * l.r.C * 2 * 2 * 2 * 4 * l.r.nq) * sizeof(uint4), st);
+  cudaMemsetAsync(l.r.halo - kResStop, 0, (kResStop + (size_t)shots * l.r.C * 2 * 2 * 2 * 4 * l.r.nq) * sizeof(uint4), st);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(shots * l.r.C);
   cfg.blockDim = dim3(l.r.nA + l.r.nR);
