@@ -143,7 +143,7 @@ struct swit_engine {
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
   // resident time loops (kernels_resident.cuh), where the split fits the device; else the variant's kernels
   ResLoop *resf = nullptr, *resb = nullptr, *resx = nullptr;  // forward, reverse, exact adjoint's reverse
-  uint4* d_halo = nullptr;  // a launch's stop word, then (from kResStop) its halo packets
+  uint4* d_halo = nullptr;  // a launch's halo packets, then its stop word
   int wait_err = 0;         // error word that a call has reported and swit_check has not
 };
 
@@ -2166,13 +2166,14 @@ static int res_setup(swit_engine* e, const swit_desc* d) {
   if (e->ckpt_k && !e->exact && !(f.ok && b.ok)) return 0;
   const size_t n = std::max(std::max(res_halo_packets(f), res_halo_packets(b)), res_halo_packets(x));
   if (!n) return 0;
-  if (int rc = dalloc(e, &e->d_halo, n + kResStop)) return rc;
+  if (int rc = dalloc(e, &e->d_halo, n + 1)) return rc;
   unsigned wait = kResWaitLimit;
   if (const char* v = std::getenv("SWIT_RES_WAIT_POLLS")) {  // a shorter wait, e.g. to test the timeout path
     const long long w = std::atoll(v);
     if (w >= 0 && w < (long long)kResWaitLimit) wait = (unsigned)w;
   }
-  f.r.halo = b.r.halo = x.r.halo = e->d_halo + kResStop;
+  f.r.halo = b.r.halo = x.r.halo = e->d_halo;
+  for (ResLoop* l : {&f, &b, &x}) l->r.stop = (int)res_halo_packets(*l);
   f.r.err = b.r.err = x.r.err = e->d_err;
   f.r.wait = b.r.wait = x.r.wait = wait;
   if (f.ok) e->resf = new ResLoop(f);

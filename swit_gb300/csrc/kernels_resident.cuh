@@ -61,8 +61,6 @@ namespace swit {
 enum { kResFwd = 0, kResAdj = 1, kResRec = 2 };
 constexpr unsigned kResWaitLimit = 1u << 22;  // polls of one halo wait
 constexpr int kResErr = 0x200;                // error word of a halo wait that gave up
-constexpr int kResStop = 8;                   // packets the stop word takes before the halo's: 128 bytes, so that
-                                              // the row tiles of a packet number stay aligned
 
 // Split of a shot over its bands and threads, and the float4 indices of the
 // shared-memory arrays.  Filled on the host (res_plan).  A slot numbers the row
@@ -81,7 +79,8 @@ struct ResPlan {
   int nside;     // side arrays a band may hold: 6, or the 3 of one side
   float negz;    // -0 (see f2)
   unsigned wait; // polls before a halo wait gives up
-  uint4* halo;   // packets: [block][role][side][parity][packet][row tile]; the stop word lies kResStop before
+  uint4* halo;   // packets: [block][role][side][parity][packet][row tile]; then the stop word
+  int stop;      // packets before the stop word
   int* err;      // the engine's error word
   // A thread's data lies together at an odd stride of float4: addresses are a base and a constant, and the
   // 16-byte accesses of a warp are free of bank conflicts.
@@ -229,7 +228,7 @@ __device__ __forceinline__ void halo_wait(const uint4* p, unsigned tag, const Re
   for (unsigned n = 0;; ++n) {
     halo_issue(p, r.nq, h);
     if (halo_here(h, tag) || dead) return;
-    int* stop = reinterpret_cast<int*>(r.halo - kResStop);
+    int* stop = reinterpret_cast<int*>(r.halo + r.stop);
     if (n >= r.wait || ((n & 255u) == 255u && *(volatile int*)stop != 0)) {
       atomicExch(stop, 1);
       atomicCAS(r.err, 0, kResErr);

@@ -194,6 +194,8 @@ inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
   }
 }
 
+// Packets of a full launch, and the stop word's behind them: with it in front, 16 or 128 bytes into the
+// allocation, some loops took 7 to 14 % longer (forward step of 2 shots 172x52 1.80 against 1.58 us).
 inline size_t res_halo_packets(const ResLoop& l) {
   return l.ok ? (size_t)l.shots * l.r.C * 2 * 2 * 2 * 4 * l.r.nq : 0;
 }
@@ -206,9 +208,9 @@ inline const ResInst& res_inst(ResKind kind, const ResLoop& l) {
   return I[0];
 }
 
-// Launch configuration of `shots` shots; the packets' tags and the stop word before them start from zero.
+// Launch configuration of `shots` shots; the packets' tags and the stop word start from zero.
 inline cudaLaunchConfig_t res_config(const ResLoop& l, int shots, cudaStream_t st, cudaLaunchAttribute* at) {
-  cudaMemsetAsync(l.r.halo - kResStop, 0, (kResStop + (size_t)shots * l.r.C * 2 * 2 * 2 * 4 * l.r.nq) * sizeof(uint4), st);
+  cudaMemsetAsync(l.r.halo, 0, (l.r.stop + 1) * sizeof(uint4), st);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(shots * l.r.C);
   cfg.blockDim = dim3(l.r.nA + l.r.nR);
