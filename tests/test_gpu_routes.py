@@ -18,6 +18,8 @@ def problem(nx, nz, npml, ns, nt):
     (dict(kernel="vec"), (481, 141, 40, 5), 3, 3),
     (dict(kernel="vec"), (1460, 716, 50, 9), 3, 2),
     (dict(kernel="vec"), (1131, 1141, 23, 4), 2, 2),
+    (dict(kernel="vec"), (1273, 1104, 24, 10), 2, 2),
+    (dict(kernel="vec"), (2001, 601, 60, 3), 3, 2),
     (dict(kernel="vec"), (1884, 896, 57, 7), 2, 1),
     (dict(kernel="vec"), (1915, 2337, 22, 3), 1, 3),
     (dict(kernel="vec", graph_branches=3), (1884, 896, 57, 4), 3, 3),
