@@ -292,8 +292,9 @@ int swit_misfit_l2(swit_engine* e, const float* src, const float* obs, double* m
  * A multi-instance engine holds n regular engines (one swit_desc each: FP32,
  * batched path, vec kernels, boundary saving; grids, shot counts and nt may all
  * differ) and steps them together: the (instance, shot) pairs are grouped
- * into L2-sized waves (an instance's own shots, or several small instances;
- * instances whose time loops fit the device as resident loops run those instead),
+ * into L2-sized waves (an instance's own shots, or several small instances; a
+ * loop that fits the device as a resident loop in every switched-on instance
+ * runs those instead),
  * and per wave each time step launches the phase kernels once over every pair
  * still running; the waves run on concurrent branches, and a call runs only
  * the waves holding a switched-on instance (swit_multi_misfit_l2's `active`).

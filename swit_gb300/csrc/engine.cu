@@ -1752,7 +1752,6 @@ struct swit_multi {
     cudaGraphExec_t g[3] = {nullptr, nullptr, nullptr};  // its forward (no strips, strips) and reverse loops
   };
   std::vector<Wave> waves;
-  std::vector<int> res_rows;  // table rows of the instances that run their resident loops
   size_t graph_nodes = size_t(1) << 20;  // kernel nodes per loop held in the waves' graphs, at most
   int branches = 3;
   cudaStream_t cap = nullptr, capx[2] = {nullptr, nullptr};
@@ -1783,11 +1782,14 @@ void multi_release(swit_multi* m) {
   }
 }
 
-// Instances whose two loops are resident run those, one launch per group of shots, spread over the branch
-// streams: the device schedules a cooperative launch whole, when its blocks fit beside those running, so
-// small problems share it.  6 uneven problems of up to 12 shots 701x251 (gradient): 177.9 ms in waves of the
-// step kernels, 125.7 ms with their resident loops.
-inline bool multi_resident(const swit_engine* e) { return e->resf && e->resb; }
+// A loop whose switched-on instances all have a resident split runs those, one launch per group of shots, spread
+// over the branch streams: the device schedules a cooperative launch whole, when its blocks fit beside those
+// running, so small problems share it.  Otherwise all run in
+// waves: a cooperative launch waits until the waves beside it leave the device enough room, and both lose.  505
+// random sets of 3 to 7 problems up to 701x400 (gradients, against waves only): 1.09 to 4.4 times as fast where
+// everything fits; 0.81 to 1.29 with the instances that fit beside waves of the others (3 problems up to
+// 619x331, 14 shots: 62.6 ms, 50.9 in waves).
+inline const ResLoop* multi_res(const swit_engine* e, int which) { return which < 2 ? e->resf : e->resb; }
 
 // Instance table, padded task lists, waves with their block tables and active
 // prefixes.  A wave's reverse-loop state stays under 0.7 L2 / branches (as the
@@ -1867,6 +1869,9 @@ int multi_build(swit_multi* m) {
     const long long v = std::atoll(gn);
     if (v >= 0) m->graph_nodes = (size_t)v;
   }
+  bool in_waves = false;  // else no call needs a wave
+  for (const swit_engine* e : m->eng)
+    for (int which = 0; which < 3; ++which) in_waves = in_waves || !multi_res(e, which);
   // A problem's shots form waves of their own, equal parts of at most budget / state shots (so that its
   // waves run its single-instance kernels; fewer, larger waves than the engine's own batches, which spread
   // one problem over the branches); problems whose shots all fit in half the budget share waves with the
@@ -1875,10 +1880,7 @@ int multi_build(swit_multi* m) {
   double used = 0.0;
   for (int r = 0; r < n; ++r) {
     const int ns = m->eng[m->order[r]]->ns;
-    if (multi_resident(m->eng[m->order[r]])) {  // no wave: its loops are launches of their own
-      m->res_rows.push_back(r);
-      continue;
-    }
+    if (!in_waves) break;
     if (ns * state[r] <= 0.5 * budget) {
       if (used + ns * state[r] > budget && !shared.back().empty()) {
         shared.emplace_back();
@@ -1949,7 +1951,7 @@ int multi_build(swit_multi* m) {
     CK(cudaMalloc(&m->d_blocks[k], std::max<size_t>(B[k].size(), 1) * sizeof(uint2)));
     CK(cudaMemcpy(m->d_blocks[k], B[k].data(), B[k].size() * sizeof(uint2), cudaMemcpyHostToDevice));
   }
-  m->branches = std::max(1, std::min(m->branches, (int)(m->waves.size() + m->res_rows.size())));
+  m->branches = std::max(1, std::min(m->branches, std::max(n, (int)m->waves.size())));
   CK(cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking));
   for (int i = 0; i < 2; ++i) {
     CK(cudaStreamCreateWithFlags(&m->capx[i], cudaStreamNonBlocking));
@@ -2001,8 +2003,20 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
   std::vector<int> rows(m->eng.size());
   for (size_t r = 0; r < rows.size(); ++r) rows[r] = on[m->order[r]];
   CK(cudaMemcpyAsync(m->d_on, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-  std::vector<int> active;
-  for (int wi = 0; wi < (int)m->waves.size(); ++wi)
+  // (work, row) of the switched-on instances, most work first, if the loop is resident in all of them
+  std::vector<std::pair<double, int>> res;
+  bool resident = true;
+  for (size_t r = 0; r < rows.size() && resident; ++r) {
+    if (!rows[r]) continue;
+    const swit_engine* e = m->eng[m->order[r]];
+    const ResLoop* l = multi_res(e, which);
+    resident = l != nullptr;
+    if (l) res.emplace_back(l->us * (e->nt - 1), (int)r);
+  }
+  if (!resident) res.clear();
+  std::stable_sort(res.begin(), res.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  std::vector<int> active;  // waves
+  for (int wi = 0; wi < (int)m->waves.size() && !resident; ++wi)
     for (int r : m->waves[wi].rows)
       if (rows[r]) {
         active.push_back(wi);
@@ -2025,15 +2039,7 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
       return fail(SWIT_E_CUDA, "multi-instance graph: %s", cudaGetErrorString(rc));
     }
   }
-  // (work, row) of the switched-on instances with resident loops, most work first
-  std::vector<std::pair<double, int>> res;
-  for (int r : m->res_rows)
-    if (rows[r]) {
-      const swit_engine* e = m->eng[m->order[r]];
-      res.emplace_back((which < 2 ? e->resf : e->resb)->us * (e->nt - 1), r);
-    }
-  std::stable_sort(res.begin(), res.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-  // the waves on the branch streams, forked from and joined back to st
+  // the resident loops or the waves on the branch streams, forked from and joined back to st
   const int br = std::max(1, std::min(m->branches, (int)(active.size() + res.size())));
   auto branch = [&](int b) { return b ? m->capx[b - 1] : st; };
   CK(cudaEventRecord(m->ev_fork, st));
@@ -2052,8 +2058,6 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
     else
       res_backward(e, *e->resb, 0, e->ns, branch(b), e->nt, 2);
   }
-  // waves count on from an even load: their work is in other units, and few calls hold both
-  if (!res.empty()) std::fill(load.begin(), load.end(), 0.0);
   for (int wi : by_work) {
     const int b = (int)(std::min_element(load.begin(), load.end()) - load.begin());
     load[b] += m->waves[wi].work;

@@ -284,8 +284,8 @@ class MultiEngine:
     differ) stepped together: (problem, shot) pairs in L2-sized waves (a
     problem's own shots, or several small problems) on concurrent branches, per
     wave one launch of each phase kernel per time step over the pairs still
-    running (swit_multi_*); problems whose time loops fit the device as resident
-    loops run those on the branches instead.  ``problems`` is a list
+    running (swit_multi_*); a loop that fits the device as a resident loop in every
+    problem switched on runs those on the branches instead.  ``problems`` is a list
     of Engine keyword dicts (nx, nz, npml, nt, dx, dt, src_xz, rec_xz[, ng,
     free_surface, block_x]); ``engines[i]`` is problem i's Engine (set_model,
     forward, ... work on it alone)."""

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from swit_gb300 import Engine, survey
+from swit_gb300 import Engine, SwitError, survey
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +45,32 @@ def test_loops_on_different_branches_match_one_branch():
             out.append((e.forward(src, save_boundary=False), e.forward(src, save_boundary=True), *e.backward(adj)))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_multi_engine_runs_waves_for_all_where_one_instance_needs_them(monkeypatch):
+    """With 0 polls any resident loop with a halo fails: beside an instance on the step kernels nothing runs
+    resident, and every result is the instance's own."""
+    from swit_gb300 import MultiEngine
+    probs = [problem(*shape, nt=nt) for shape, nt in (((60, 40, 12, 2), 60), ((52, 36, 10, 3), 80), ((40, 30, 8, 1), 50))]
+    obss = [np.random.default_rng(i).standard_normal((s.ns, s.ng, s.nt)).astype(np.float32) * np.float32(1e-3)
+            for i, (s, _, _) in enumerate(probs)]
+    want = []
+    for (s, src, rho), o in zip(probs, obss):
+        with Engine(**s.engine_args()) as e:
+            e.set_model(s.vp_true, rho)
+            want.append((e.gradient_l2(src, o), e.misfit_l2(src, o)))
+    for k, v in (("SWIT_RES_WAIT_POLLS", "0"), ("SWIT_RES_FWD_TILES", "1"), ("SWIT_RES_BWD_TILES", "1")):
+        monkeypatch.setenv(k, v)
+    srcs = [src for _, src, _ in probs]
+    with MultiEngine([dict(s.engine_args(), kernel=k) for (s, _, _), k in zip(probs, ("auto", "vec", "auto"))]) as m:
+        for e, (s, _, rho) in zip(m.engines, probs):
+            e.set_model(s.vp_true, rho)
+        got = m.gradient_l2(srcs, obss)
+        every = m.misfit_l2(srcs, obss)
+        with pytest.raises(SwitError, match="SWIT_E_TIMEOUT"):  # the two others run resident
+            m.misfit_l2(srcs, obss, active=[True, False, True])
+    for g, (w, _) in zip(got, want):
+        for k in ("grad", "illum_fw", "illum_bk"):
+            np.testing.assert_array_equal(g[k], w[k])
+        assert g["misfit"] == w["misfit"]
+    assert every == [v for _, v in want]
