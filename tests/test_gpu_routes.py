@@ -74,3 +74,41 @@ def test_multi_engine_runs_waves_for_all_where_one_instance_needs_them(monkeypat
             np.testing.assert_array_equal(g[k], w[k])
         assert g["misfit"] == w["misfit"]
     assert every == [v for _, v in want]
+
+
+@pytest.mark.parametrize("env", [{}, {"SWIT_MULTI_WAVE_BYTES": "1"}, {"SWIT_MULTI_WAVE_BYTES": "5e5"},
+                                 {"SWIT_MULTI_WAVE_BYTES": "1", "SWIT_MULTI_GRAPH_NODES": "0"},
+                                 {"SWIT_MULTI_WAVE_BYTES": "5e5", "SWIT_MULTI_GRAPH_NODES": "0"},
+                                 {"SWIT_MULTI_WAVE_BYTES": "1", "SWIT_MULTI_GRAPH_NODES": "700"}])
+def test_multi_engine_waves_of_step_kernels_match_resident_engines(env, monkeypatch):
+    """Every wave layout on the step kernels (kernel="vec": nothing resident), also after a partial call, against
+    the problems' own engines on the default kernels."""
+    import torch
+    from swit_gb300 import MultiEngine
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    probs = [survey.small(nx=nx, nz=nz, npml=npml, nt=nt, dx=dx, ns=ns, seed=seed) for nx, nz, npml, nt, dx, ns, seed in
+             ((52, 30, 10, 260, 10.0, 3, 3), (40, 36, 8, 180, 12.0, 2, 4), (64, 24, 9, 320, 10.0, 4, 5))]
+    srcs, obss, want = [s.source() for s in probs], [], []
+    for s, x in zip(probs, srcs):
+        with Engine(**s.engine_args()) as e:
+            assert e.query()["kernel"] == "resident"
+            e.set_model(s.vp_true, s.rho(s.vp_true))
+            obss.append(e.forward(x, save_boundary=False))
+            e.set_model(s.vp_init, s.rho(s.vp_true))
+            want.append(e.gradient_l2(x, obss[-1]))
+    with MultiEngine([dict(s.engine_args(), kernel="vec") for s in probs]) as m:
+        for e, s in zip(m.engines, probs):
+            assert e.query()["kernel"] == "vec"
+            e.set_model(s.vp_init, s.rho(s.vp_true))
+        outs = [m.gradient_l2(srcs, obss), m.gradient_l2(srcs, obss)]
+        assert m.misfit_l2(srcs, obss) == [w["misfit"] for w in want]
+        assert m.misfit_l2(srcs, obss, active=[False, True, False]) == [0.0, want[1]["misfit"], 0.0]
+        outs.append(m.gradient_l2(srcs, obss))
+        outs.append([{k: v.cpu().numpy() if torch.is_tensor(v) else v for k, v in o.items()} for o in
+                     m.gradient_l2([torch.from_numpy(x).cuda() for x in srcs], [torch.from_numpy(x).cuda() for x in obss])])
+    for out in outs:
+        for g, w in zip(out, want):
+            for k in ("grad", "illum_fw", "illum_bk"):
+                np.testing.assert_array_equal(g[k], w[k])
+            assert g["misfit"] == w["misfit"]
