@@ -141,8 +141,10 @@ struct swit_engine {
   void *xm = nullptr, *xsrc = nullptr, *xdadc = nullptr;
   std::vector<cudaGraphExec_t> gxb;
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
-  // resident time loops (kernels_resident.cuh), where the split fits the device; else the variant's kernels
-  ResLoop *resf = nullptr, *resb = nullptr, *resx = nullptr;  // forward, reverse, exact adjoint's reverse
+  // resident time loops (kernels_resident.cuh), where a split fits the device and is faster (ResLoop::alone); else
+  // the variant's kernels: forward (0) and saving forward (1), reverse, exact adjoint's reverse.  An instance of a
+  // multi-instance engine keeps every loop that fits
+  ResLoop *resf[2] = {nullptr, nullptr}, *resb = nullptr, *resx = nullptr;
   uint4* d_halo = nullptr;  // a launch's halo packets, then its stop word
   int wait_err = 0;         // error word that a call has reported and swit_check has not
 };
@@ -240,11 +242,14 @@ inline Sources make_src(const swit_engine* e) { return Sources{e->d_isx, e->d_is
 #include "resident_host.cuh"
 namespace {
 
+// A loop as the engine by itself runs it: null where it takes the variant's kernels.
+inline const ResLoop* res_alone(const ResLoop* l) { return l && l->alone ? l : nullptr; }
+
 void res_free(swit_engine* e) {
-  delete e->resf;
-  delete e->resb;
-  delete e->resx;
-  e->resf = e->resb = e->resx = nullptr;
+  for (ResLoop** l : {&e->resf[0], &e->resf[1], &e->resb, &e->resx}) {
+    delete *l;
+    *l = nullptr;
+  }
 }
 
 // Launch shape of the stencil kernels for a batch of nb shots.
@@ -369,7 +374,7 @@ void launch_forward_steps(swit_engine* e, bool store, int shot0, int nb, cudaStr
                           int it_hi = -1, bool res = false) {
   if (it_hi < 0) it_hi = e->nt;
   if (res) {
-    res_forward(e, *e->resf, store, shot0, nb, st, it_lo, it_hi);
+    res_forward(e, *e->resf[store], store, shot0, nb, st, it_lo, it_hi);
     return;
   }
   if (e->variant == 4 || e->variant == 5) {
@@ -724,8 +729,7 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  // the exact adjoint's forward keeps D of every step in its reverse loop's layout
-  if (e->resf && !(store && e->exact && !e->ckpt_k && !e->resx)) {
+  if (res_alone(e->resf[store && !e->ckpt_k])) {
     if (store && e->ckpt_k)
       forward_checkpointed<R>(e, 0, e->ns, st, true);
     else
@@ -762,7 +766,7 @@ int run_backward_loop(swit_engine* e, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  if (e->resb) {
+  if (res_alone(e->resb)) {
     if (e->ckpt_k)
       backward_checkpointed<R>(e, 0, e->ns, st, true);
     else
@@ -880,7 +884,7 @@ int run_exact_loop(swit_engine* e, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  if (e->resx) {
+  if (res_alone(e->resx)) {
     exact_reverse<R>(e, 0, e->ns, st, true);
     CK(cudaGetLastError());
     return 0;
@@ -1279,7 +1283,7 @@ int profile_resident(swit_engine* e, int32_t launches[4], double mean_ms[4], cud
   for (void* q : {e->p, e->u, e->w, e->pb, e->ub, e->wb, e->pe, e->ue, e->we, e->dg, e->dfw, e->dbk})
     CK(cudaMemsetAsync(q, 0, fb, st));
   std::vector<cudaEvent_t> ev[2];
-  res_forward(e, *e->resf, true, 0, e->ns, st, 2, e->nt, &ev[0]);
+  res_forward(e, *e->resf[1], true, 0, e->ns, st, 2, e->nt, &ev[0]);
   res_backward(e, *e->resb, 0, e->ns, st, e->nt, 2, &ev[1]);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(st));
@@ -1303,7 +1307,7 @@ template <class R>
 int profile_impl(swit_engine* e, int32_t launches[4], double mean_ms[4], cudaStream_t st) {
   if (e->ckpt_k) return fail(SWIT_E_STATE, "this call needs boundary saving (checkpoint_every = 0)");
   if constexpr (sizeof(R) == 4)
-    if (e->resf && e->resb) return profile_resident(e, launches, mean_ms, st);
+    if (res_alone(e->resf[1]) && res_alone(e->resb)) return profile_resident(e, launches, mean_ms, st);
   if (e->variant == 3 && e->path == 0) return profile_vec_graphs<R>(e, launches, mean_ms, st);
   Grid<R> g = make_grid<R>(e);
   const int nshot_launch = e->path == 1 ? 1 : e->batch;
@@ -1784,12 +1788,12 @@ void multi_release(swit_multi* m) {
 
 // A loop whose switched-on instances all have a resident split runs those, one launch per group of shots, spread
 // over the branch streams: the device schedules a cooperative launch whole, when its blocks fit beside those
-// running, so small problems share it.  Otherwise all run in
+// running, so small problems share it, also those that would take the step kernels alone.  Otherwise all run in
 // waves: a cooperative launch waits until the waves beside it leave the device enough room, and both lose.  505
 // random sets of 3 to 7 problems up to 701x400 (gradients, against waves only): 1.09 to 4.4 times as fast where
 // everything fits; 0.81 to 1.29 with the instances that fit beside waves of the others (3 problems up to
 // 619x331, 14 shots: 62.6 ms, 50.9 in waves).
-inline const ResLoop* multi_res(const swit_engine* e, int which) { return which < 2 ? e->resf : e->resb; }
+inline const ResLoop* multi_res(const swit_engine* e, int which) { return which < 2 ? e->resf[which] : e->resb; }
 
 // Instance table, padded task lists, waves with their block tables and active
 // prefixes.  A wave's reverse-loop state stays under 0.7 L2 / branches (as the
@@ -2054,7 +2058,7 @@ int multi_loop(swit_multi* m, int which, const std::vector<int>& on, cudaStream_
     load[b] += q.first;
     swit_engine* e = m->eng[m->order[q.second]];
     if (which < 2)
-      res_forward(e, *e->resf, which == 1, 0, e->ns, branch(b), 2, e->nt);
+      res_forward(e, *e->resf[which], which == 1, 0, e->ns, branch(b), 2, e->nt);
     else
       res_backward(e, *e->resb, 0, e->ns, branch(b), e->nt, 2);
   }
@@ -2156,22 +2160,47 @@ void auto_batches(swit_engine* e, int branches) {
 }
 
 // Resident time loops for FP32 engines on the default kernels and launch
-// shapes, where a split fits the device.  A checkpointed engine runs both loops
-// segment by segment over all shots, so it takes them only together and for
-// segments long enough to pay for loading and storing the state (10 shots
-// 801x301, 200 steps: 18.0 against 16.9 ms at 12 steps per segment, 16.0 against
-// 16.5 at 16; 2 shots 182x84, 378 steps: 4.5 against 7.9 at 16); vx adjoint
-// sources change u between the phases, also in the columns a band recomputes,
-// which the resident reverse loop does not do.
-static int res_setup(swit_engine* e, const swit_desc* d) {
+// shapes, each where a split fits the device and its estimate is below the vec
+// kernels' (reverse of 23 shots 587x238, one shot per launch: 67.6 resident, 51.1
+// vec; forward of 3 shots 1350x660: 16.5 and 13.4; of one: 5.5 and 7.8).  Two
+// loops go together where they run as one: the exact adjoint's saving forward and
+// reverse (D lies in tiles), and a checkpointed run's, which alternate segment by
+// segment over all shots and pay for launches and state at every segment (10
+// shots 801x301, 200 steps: 18.0 against 16.9 ms at 12 steps per segment, 16.0
+// against 16.5 at 16).  vx adjoint sources change u between the phases, also in
+// the columns a band recomputes, which the resident reverse loop does not do.
+static int res_setup(swit_engine* e, const swit_desc* d, bool multi) {
   if (d->kernel_variant || e->prec || e->path || d->shots_per_batch || d->graph_branches || d->block_x) return 0;
   if (e->ckpt_k && e->ckpt_k < 16) return 0;
-  ResLoop f, b, x;
-  res_choose(e, kResLoopFwd, f);
-  if (!e->exact && e->rcomp != 1) res_choose(e, kResLoopBwd, b);
-  if (e->exact && !e->rcomp && f.ok) res_choose(e, kResLoopXadj, x);
-  if (e->ckpt_k && !e->exact && !(f.ok && b.ok)) return 0;
-  const size_t n = std::max(std::max(res_halo_packets(f), res_halo_packets(b)), res_halo_packets(x));
+  const int steps = e->ckpt_k ? e->ckpt_k : e->nt - 1;
+  const ResKind rev = e->exact ? kResLoopXadj : kResLoopBwd;
+  ResLoop f, s, b;
+  res_choose(e, kResLoopFwd, steps, multi, f);
+  res_choose(e, kResLoopSave, steps, multi, s);
+  if (e->exact ? !e->rcomp : e->rcomp != 1) res_choose(e, rev, steps, multi, b);
+  // whether loops of the given kinds, run together, are the faster ones
+  auto keep = [&](std::initializer_list<std::pair<ResKind, ResLoop*>> loops) {
+    double res = 0.0, vec = 0.0;
+    bool ok = true, forced = false;
+    for (const auto& l : loops) {
+      ok = ok && l.second->ok;
+      forced = forced || res_forced(l.first);
+      res += l.second->us;
+      vec += vec_step_us(e, l.first);
+    }
+    for (const auto& l : loops) {
+      l.second->alone = ok && (forced || res < vec);
+      l.second->ok = l.second->alone || (multi && l.second->ok);
+    }
+  };
+  keep({{kResLoopFwd, &f}});
+  if (e->exact || e->ckpt_k) {
+    keep({{kResLoopSave, &s}, {rev, &b}});
+  } else {
+    keep({{kResLoopSave, &s}});
+    keep({{rev, &b}});
+  }
+  const size_t n = std::max(std::max(res_halo_packets(f), res_halo_packets(s)), res_halo_packets(b));
   if (!n) return 0;
   if (int rc = dalloc(e, &e->d_halo, n + 1)) return rc;
   unsigned wait = kResWaitLimit;
@@ -2179,17 +2208,21 @@ static int res_setup(swit_engine* e, const swit_desc* d) {
     const long long w = std::atoll(v);
     if (w >= 0 && w < (long long)kResWaitLimit) wait = (unsigned)w;
   }
-  f.r.halo = b.r.halo = x.r.halo = e->d_halo;
-  for (ResLoop* l : {&f, &b, &x}) l->r.stop = (int)res_halo_packets(*l);
-  f.r.err = b.r.err = x.r.err = e->d_err;
-  f.r.wait = b.r.wait = x.r.wait = wait;
-  if (f.ok) e->resf = new ResLoop(f);
-  if (b.ok) e->resb = new ResLoop(b);
-  if (x.ok) e->resx = new ResLoop(x);
+  auto take = [&](ResLoop& l, ResLoop*& at) {
+    if (!l.ok) return;
+    l.r.halo = e->d_halo;
+    l.r.stop = (int)res_halo_packets(l);
+    l.r.err = e->d_err;
+    l.r.wait = wait;
+    at = new ResLoop(l);
+  };
+  take(f, e->resf[0]);
+  take(s, e->resf[1]);
+  take(b, e->exact ? e->resx : e->resb);
   return 0;
 }
 
-int swit_create(const swit_desc* d, swit_engine** out) {
+static int create_engine(const swit_desc* d, swit_engine** out, bool multi) {
   if (!d || !out) return fail(SWIT_E_ARG, "null argument");
   *out = nullptr;
   if (d->nx < 8 || d->nz < 8) return fail(SWIT_E_ARG, "nx and nz must be >= 8 (got %d, %d)", d->nx, d->nz);
@@ -2482,7 +2515,7 @@ int swit_create(const swit_desc* d, swit_engine** out) {
       return rc;
     }
   }
-  rc = res_setup(e, d);
+  rc = res_setup(e, d, multi);
   if (rc) {
     release(e);
     delete e;
@@ -2517,13 +2550,15 @@ int swit_create(const swit_desc* d, swit_engine** out) {
   e->launches_fwd = (e->variant == 4 || e->variant == 5) ? fwaves : per * (e->nt - 1) * per_step;
   e->launches_bwd = e->variant == 4 ? per : per * (e->nt - 1) * per_step * (e->ckpt_k ? 2 : 1);
   const int segs = std::max(1, e->ckpt_m);
-  const int resf = e->resf ? segs * ((ns + e->resf->shots - 1) / e->resf->shots) : 0;
-  if (e->resf && !(e->exact && !e->ckpt_k && !e->resx)) e->launches_fwd = resf;
-  if (const ResLoop* l = e->resb ? e->resb : e->resx)
-    e->launches_bwd = segs * ((ns + l->shots - 1) / l->shots) + (e->ckpt_k ? resf : 0);
+  auto res_launches = [&](const ResLoop* l) { return segs * ((ns + l->shots - 1) / l->shots); };
+  if (const ResLoop* l = res_alone(e->resf[!e->ckpt_k])) e->launches_fwd = res_launches(l);
+  if (const ResLoop* l = res_alone(e->resb ? e->resb : e->resx))
+    e->launches_bwd = res_launches(l) + (e->ckpt_k ? res_launches(e->resf[1]) : 0);
   *out = e;
   return 0;
 }
+
+int swit_create(const swit_desc* d, swit_engine** out) { return create_engine(d, out, false); }
 
 int swit_set_model(swit_engine* e, const float* vp, const float* rho, int on_device, void* stream) {
   if (!e || !vp || !rho) return fail(SWIT_E_ARG, "null argument");
@@ -2670,7 +2705,7 @@ int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_b
   if (block_x) *block_x = e->bx;
   if (kernels_per_forward) *kernels_per_forward = e->launches_fwd;
   if (kernels_per_backward) *kernels_per_backward = e->launches_bwd;
-  if (kernel_variant) *kernel_variant = e->resf && (e->resb || e->resx) ? 7 : e->variant;
+  if (kernel_variant) *kernel_variant = res_alone(e->resf[1]) && res_alone(e->resb ? e->resb : e->resx) ? 7 : e->variant;
   return 0;
 }
 
@@ -2678,8 +2713,7 @@ int swit_query_loop(const swit_engine* e, int32_t loop, int32_t* kernel_variant,
                     int32_t* branches) {
   if (!e) return fail(SWIT_E_ARG, "null argument");
   if (loop < 0 || loop > 2) return fail(SWIT_E_ARG, "loop must be 0 (forward), 1 (saving forward) or 2 (reverse) (got %d)", loop);
-  const ResLoop* l = loop == 2 ? (e->exact ? e->resx : e->resb) : e->resf;
-  if (loop == 1 && e->exact && !e->ckpt_k && !e->resx) l = nullptr;
+  const ResLoop* l = res_alone(loop == 2 ? (e->exact ? e->resx : e->resb) : e->resf[loop]);
   const int batch = e->path == 1 ? 1 : (loop == 2 ? e->batch : fwd_batch(e));
   const int br = e->path == 1 ? 1 : std::min(loop == 2 ? e->branches : e->fbranches, (e->ns + batch - 1) / batch);
   if (kernel_variant) *kernel_variant = l ? 7 : e->variant;
@@ -2733,7 +2767,7 @@ int swit_multi_create(const swit_desc* descs, int32_t n, swit_multi** out) {
   swit_multi* m = new swit_multi();
   for (int i = 0; i < n; ++i) {
     swit_engine* e = nullptr;
-    int rc = swit_create(&descs[i], &e);
+    int rc = create_engine(&descs[i], &e, true);
     if (rc) {
       std::string msg = g_err;
       multi_release(m);

@@ -6,9 +6,10 @@
 // it is compiled for), its split and the shots of one launch.
 struct ResLoop {
   bool ok = false;
+  bool alone = false;  // runs where the engine runs by itself
   int tx = 0, maxt = 0;
   int shots = 0;  // per launch, at most
-  double us = 0.0;  // estimated microseconds per time step of all shots
+  double us = 0.0;  // estimated microseconds per time step of all shots, launches included
   swit::ResPlan r{};
 };
 
@@ -21,7 +22,8 @@ using ResBwdFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, const float*
 
 using ResXadjFn = void (*)(Grid<float>, ResPlan, Sources, Receivers, XAdj<float>, int, int, int);
 
-enum ResKind { kResLoopFwd, kResLoopBwd, kResLoopXadj };
+// A saving forward keeps the strips, or the divergence for the exact adjoint.
+enum ResKind { kResLoopFwd, kResLoopSave, kResLoopBwd, kResLoopXadj };
 
 struct ResInst {
   int tx, maxt;
@@ -37,7 +39,7 @@ inline const ResInst* res_instances(ResKind kind, int& n) {
                               {4, 384, nullptr, nullptr, k_bwd_res<4, 384>, nullptr}};
   static const ResInst X[] = {{4, 384, nullptr, nullptr, nullptr, k_xadj_res<4, 384>}};
   n = kind == kResLoopXadj ? 1 : 2;
-  return kind == kResLoopFwd ? F : (kind == kResLoopBwd ? B : X);
+  return kind <= kResLoopSave ? F : (kind == kResLoopBwd ? B : X);
 }
 
 // Split of a shot into bands of at most `tiles` column tiles, with the shared memory of a block.
@@ -52,7 +54,7 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
   r.m0 = e->L / tx;
   r.m1 = (e->L + e->nx - 1) / tx;
   // a band reaches the strip columns of both sides only if it is nearly as wide as the interior; with 4 columns
-  // per thread there is room for both, and a constant index (481x141: 14.1 against 14.3 us per step)
+  // per thread there is room for both, and a constant index
   r.nside = tx == 4 || r.W + 8 >= e->nx ? 6 : 3;
   if (bwd) {
     r.kr = (e->fs - 2 + 3) / 4;  // rows from fs-1-4 kr <= 1
@@ -124,35 +126,84 @@ inline ResPlan res_plan(const swit_engine* e, ResKind kind, int tx, int tiles) {
   return r;
 }
 
-// Estimated microseconds of one time step of a launch whose fullest SM holds `bpsm` blocks, fitted to
-// measured steps (GB300, 11 grids of 60x40 to 700x40 and 401x151 in bands of 1 to 10 column tiles, 1 to 15
-// warps per block): a fixed part, the dependent chain of a step (updates, barriers, halo), and a part by the
-// warps that share the SM.  Bands of one column tile exchange both edges in the same threads, and in bands of
-// two every thread has an edge (forward of 101x51: 2.00 us with one tile, 2.06 with two, 1.64 with three);
-// a shot in one band exchanges nothing.  The reverse loop's 128-register instance pays for its spills; the
-// forward's with 8 columns per thread holds half as many points again per SM and is taken where that saves
-// launches (10 shots 801x301: 9.7 against 11.0 us per step in 2 and 4 launches; 49 shots 481x141: 17.9
-// against 14.2) or nothing else fits (2001x601).
-inline double res_step_us(const ResPlan& r, ResKind kind, int maxt, int bpsm, int tiles) {
-  const double warps = bpsm * ((r.nA + r.nR) / 32);
-  const double edge[3][2] = {{0.40, 0.33}, {0.50, 0.20}, {0.50, 0.37}};
-  const double t = kind == kResLoopFwd   ? 1.5 + (maxt < 512 ? 0.28 : 0.09) * warps
-                   : kind == kResLoopBwd ? 1.95 + (maxt > 384 ? 0.23 : 0.095) * warps
-                                         : 1.85 + 0.11 * warps;
-  return t + (r.C == 1 ? -0.3 : (tiles <= 2 ? edge[kind][tiles - 1] : 0.0));
+// Estimated microseconds of one time step of a launch whose fullest SM holds `bpsm` blocks: the dependent chain
+// of a step (updates, barriers, halo), a part for every warp of the SM and one for every warp of a scheduler, by
+// instance and by how a shot is split: one band, which exchanges nothing, and bands of one tile (both edges in
+// the same threads), of two (every thread has an edge) and of more.  Fitted to 10,400 measured loops (GB300,
+// 1,400 problems of 61x41 to 2000x1000, every width of band): 7 % rms.  E.g.
+// forward of 49 shots 481x141 in 5 launches (15 warps) 12.4 estimated and measured, saving 14.6 and 14.8,
+// reverse in 13 launches 35.3 and 35.5; forward of one shot 2001x601 (8 columns, 133 bands of two tiles, 11
+// warps) 5.2 and 5.2, saving 5.9 and 5.7.
+inline double res_step_us(const ResPlan& r, ResKind kind, bool exact, int tx, int maxt, int bpsm) {
+  struct Cost {
+    double a, warp, sched, least;
+  };
+  static const Cost
+      fwd4[4] = {{0.52, 0.080, 0.110, 0.0}, {1.61, 0.046, 0.174, 0.0}, {1.53, 0.045, 0.172, 0.0}, {1.25, 0.034, 0.182, 0.0}},
+      fwd8[4] = {{1.40, 0.050, 0.500, 0.0}, {2.15, 0.335, 0.000, 3.2}, {0.95, 0.390, 0.000, 3.4}, {1.60, 0.130, 0.370, 2.9}},
+      save4[4] = {{1.20, 0.090, 0.110, 0.0}, {1.95, 0.040, 0.230, 0.0}, {1.86, 0.050, 0.190, 0.0}, {1.56, 0.047, 0.164, 0.0}},
+      save8[4] = {{1.47, 0.200, 0.310, 0.0}, {3.00, 0.335, 0.000, 4.0}, {1.75, 0.380, 0.000, 4.1}, {2.60, 0.150, 0.180, 3.6}},
+      bwd384[4] = {{1.60, 0.057, 0.114, 0.0}, {2.19, 0.120, 0.069, 0.0}, {1.64, 0.087, 0.112, 0.0}, {1.69, 0.057, 0.114, 0.0}},
+      bwd512[4] = {{3.80, 0.088, 0.000, 0.0}, {3.80, 0.088, 0.000, 0.0}, {3.80, 0.088, 0.000, 0.0}, {3.80, 0.088, 0.000, 0.0}},
+      xadj[4] = {{1.50, 0.014, 0.257, 0.0}, {2.37, 0.014, 0.286, 0.0}, {2.41, 0.031, 0.158, 0.0}, {1.93, 0.014, 0.257, 0.0}};
+  const bool strips = kind == kResLoopSave && !exact;  // keeping D costs the forward next to nothing
+  const Cost* c = kind == kResLoopXadj  ? xadj
+                  : kind == kResLoopBwd ? (maxt > 384 ? bwd512 : bwd384)  // 512 threads: 128 registers, spills
+                  : tx == 8             ? (strips ? save8 : fwd8)
+                                        : (strips ? save4 : fwd4);
+  c += r.C == 1 ? 0 : std::min((r.nt_tiles + r.C - 1) / r.C, 3);
+  const int warps = bpsm * ((r.nA + r.nR) / 32);
+  const double t = std::max(c->least, c->a + c->warp * warps + c->sched * ((warps + 3) / 4));
+  return tx == 8 && bpsm > 1 ? 1.1 * t : t;
+}
+constexpr double kResLaunchUs = 20.0;  // a launch's memset, state in and out, tables
+
+// Estimated microseconds of one time step of all shots on the vec kernels, in the engine's batches and
+// branches: per launch of a branch the chain of its two kernels, per point the throughput, less of it where the
+// state in flight outgrows its share of L2.  Fitted to the loops of 425 engines, 61x41 to 2001x2337: 6 to
+// 8 % rms.  E.g. forward of 1 and 3 shots 2001x601 9.0 and 17.9 estimated, 8.5 and 19.2 measured; 23 shots
+// 587x238 23.4 and 24.9, reverse 50.9 and 51.1.
+inline double vec_step_us(const swit_engine* e, ResKind kind) {
+  const bool fwd = kind <= kResLoopSave, xadj = kind == kResLoopXadj;
+  const double pml = 1e-6 * e->NX * e->NZ, inner = 1e-6 * e->nx * e->nz;
+  const double pts = kind == kResLoopBwd ? pml + inner : 1e-6 * e->NX * (e->nz + e->L);
+  const int batch = fwd ? e->fbatch : e->batch, nl = (e->ns + batch - 1) / batch;
+  const int br = std::min(fwd ? e->fbranches : e->branches, nl);
+  const double rounds = 0.5 * ((nl + br - 1) / br + (double)nl / br);  // the last one may leave branches idle
+  const double shot = kind == kResLoopBwd ? 12.0 * pml + 24.0 * inner : (xadj ? 20.0 : 12.0) * pml;  // MB
+  const double mb = br * batch * shot + 20.0 * pml, launch = std::min(1.0, batch * pts / 0.3);
+  const double all = e->ns * pts;
+  if (xadj) return rounds * (7.0 + 0.8 * launch) + all * (6.7 + std::min(4.0, 0.040 * std::max(0.0, mb - 36.0)));
+  if (!fwd)  // both wavefields in the interior, the adjoint alone outside it
+    return rounds * (8.5 + 1.25 * launch) + e->ns * (5.5 * inner + 6.3 * (pml - inner)) +
+           all * std::min(4.5, 0.031 * std::max(0.0, mb - 74.0));
+  return rounds * ((kind == kResLoopSave ? 5.7 : 5.3) + 0.8 * launch) +
+         all * ((e->ns <= 2 ? 2.05 : 2.5) + std::min(6.0, 0.012 * std::max(0.0, mb - 60.0)));
 }
 
-// The fastest split by estimate among those whose blocks are co-resident.
-inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
+// Whether a split is set by the environment (column tiles per band; columns per thread), e.g. to test it.
+inline int res_forced_tiles(ResKind kind) {
+  const char* v = std::getenv(kind > kResLoopSave ? "SWIT_RES_BWD_TILES" : "SWIT_RES_FWD_TILES");
+  return v ? std::atoi(v) : 0;
+}
+inline int res_forced_cols(ResKind kind) {
+  const char* v = kind > kResLoopSave ? nullptr : std::getenv("SWIT_RES_FWD_COLS");
+  return v ? std::atoi(v) : 0;
+}
+inline bool res_forced(ResKind kind) { return res_forced_tiles(kind) || res_forced_cols(kind); }
+
+// The fastest split by estimate among those whose blocks are co-resident, for launches of `steps` steps.  A
+// multi-instance engine's launches share the device, so there a split that takes fewer SMs may be slower by itself
+// (reverse loops of 3, 1 and 2 shots up to 288x138: in bands that add up to 187 blocks they overlap, 3.0 ms a
+// gradient, 232 blocks do not, 4.0 ms; gradients of 505 sets of 3 to 7 problems in the mean 2.5 % faster with a
+// weight of 0.4 than of 0.1).
+inline void res_choose(const swit_engine* e, ResKind kind, int steps, bool multi, ResLoop& out) {
   int dev = 0, sms = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return;
-  int want = 0;  // column tiles per band instead of the estimate's choice, e.g. to test a split
-  if (const char* v = std::getenv(kind != kResLoopFwd ? "SWIT_RES_BWD_TILES" : "SWIT_RES_FWD_TILES")) want = std::atoi(v);
-  int cols = 0;  // columns per thread, likewise
-  if (const char* v = std::getenv("SWIT_RES_FWD_COLS")) cols = kind == kResLoopFwd ? std::atoi(v) : 0;
+  const int want = res_forced_tiles(kind), cols = res_forced_cols(kind);
   int ninst = 0;
   const ResInst* I = res_instances(kind, ninst);
   double best = 0.0;
@@ -167,10 +218,9 @@ inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
       lastC = r.C;
       if (r.nA + r.nR > I[i].maxt) break;
       if (r.smem > optin) continue;
-      const void* f = e->exact && kind == kResLoopFwd ? (const void*)I[i].fd : I[i].any();
+      const void* f = e->exact && kind == kResLoopSave ? (const void*)I[i].fd : I[i].any();
       int occ = 0;
-      if (cudaFuncSetAttribute(I[i].any(), cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
-          cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, r.nA + r.nR, r.smem) != cudaSuccess) {
         cudaGetLastError();
         continue;
@@ -180,9 +230,10 @@ inline void res_choose(const swit_engine* e, ResKind kind, ResLoop& out) {
       const int waves = (e->ns + fit - 1) / fit;
       const int shots = (e->ns + waves - 1) / waves;
       const int bpsm = (shots * r.C + sms - 1) / sms;
-      const double t = waves * res_step_us(r, kind, I[i].maxt, bpsm, (r.nt_tiles + r.C - 1) / r.C);
-      if (!out.ok || t < best) {
-        best = t;
+      const double t = waves * (res_step_us(r, kind, e->exact, I[i].tx, I[i].maxt, bpsm) + kResLaunchUs / steps);
+      const double cost = multi ? t * (1.0 + 0.4 * std::min(1.0, (double)shots * r.C / sms)) : t;
+      if (!out.ok || cost < best) {
+        best = cost;
         out.ok = true;
         out.tx = I[i].tx;
         out.maxt = I[i].maxt;

@@ -112,3 +112,60 @@ def test_multi_engine_waves_of_step_kernels_match_resident_engines(env, monkeypa
             for k in ("grad", "illum_fw", "illum_bk"):
                 np.testing.assert_array_equal(g[k], w[k])
             assert g["misfit"] == w["misfit"]
+
+
+@pytest.mark.parametrize("shape,resident", [
+    # where both fit, the faster one by a wide margin (us per step of forward, saving forward and reverse, resident
+    # and vec): 1.4, 1.8, 2.3 and 5.0, 5.4, 8.6
+    ((101, 51, 20, 1), (1, 1, 1)),
+    ((481, 141, 40, 10), (1, 1, 1)),   # 2.5, 3.0, 9.0 and 8.5, 9.0, 16
+    ((2001, 601, 60, 1), (1, 1, 0)),   # 5.2, 5.7 and 8.5, 8.9; no reverse split fits
+    ((1350, 660, 30, 1), (1, 1, 0)),   # 5.5, 5.9 and 7.8, 8.2
+    ((1350, 660, 30, 3), (0, 0, 0)),   # 16.5, 18.6 and 13.4, 13.6
+    ((691, 780, 16, 3), (0, 0, 0)),    # 12.4, 14.9 and 9.3, 9.6
+    ((587, 238, 48, 23), (1, 1, 0)),   # 10.1, 11.6, 67.6 and 24.9, 27.6, 51.1
+    ((338, 311, 51, 14), (1, 1, 0))])  # 6.7, 8.0, 40.7 and 12.0, 12.2, 23.0
+def test_resident_loops_run_where_they_are_faster(shape, resident):
+    s, _, _ = problem(*shape, nt=400)
+    with Engine(**s.engine_args()) as e:
+        got = tuple(int(e.query_loop(k)["kernel"] == "resident") for k in ("forward", "saving", "reverse"))
+        assert got == resident
+        assert e.query()["kernel"] == ("resident" if resident[1] and resident[2] else "vec")
+
+
+def test_exact_adjoint_keeps_both_loops_on_one_path():
+    """Its saving forward and its reverse loop share the layout of the stored divergence."""
+    for shape in ((241, 121, 20, 4), (687, 820, 38, 3)):
+        s, _, _ = problem(*shape, nt=40)
+        with Engine(**s.engine_args(), adjoint="exact") as e:
+            assert e.query_loop("saving")["kernel"] == e.query_loop("reverse")["kernel"] == \
+                ("resident" if s.nx == 241 else "vec")
+
+
+def test_forward_and_reverse_on_different_kernels_match_the_step_kernels():
+    s, src, rho = problem(338, 311, 51, 14, 90)
+    adj = np.random.default_rng(2).standard_normal((s.ns, s.ng, s.nt)).astype(np.float32)
+    out = []
+    for kernel in ("auto", "vec"):
+        with Engine(**s.engine_args(), kernel=kernel) as e:
+            assert [e.query_loop(k)["kernel"] for k in ("saving", "reverse")] == \
+                (["resident", "vec"] if kernel == "auto" else ["vec", "vec"])
+            e.set_model(s.vp_true, rho)
+            out.append((e.forward(src, save_boundary=True), *e.backward(adj)))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_checkpointed_forward_and_reverse_on_different_kernels_match_the_step_kernels():
+    """The forward pass leaves checkpoints that the other kernels' reverse pass starts from."""
+    s, src, rho = problem(643, 225, 53, 17, 64)
+    adj = np.random.default_rng(3).standard_normal((s.ns, s.ng, s.nt)).astype(np.float32)
+    out = []
+    for kernel in ("auto", "vec"):
+        with Engine(**s.engine_args(), kernel=kernel, checkpoint_every=21) as e:
+            assert [e.query_loop(k)["kernel"] for k in ("forward", "saving", "reverse")] == \
+                (["resident", "vec", "vec"] if kernel == "auto" else ["vec"] * 3)
+            e.set_model(s.vp_true, rho)
+            out.append((e.forward(src, save_boundary=True), *e.backward(adj)))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
