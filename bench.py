@@ -492,13 +492,15 @@ def run_mine(args):
 
     U, B = work_units(sv.nx, sv.nz, sv.npml, sv.nt, sv.ng)
     peak, peak_kind = measured_peak()
+    loops = {k: eng.query_loop(k) for k in ("saving", "reverse")}
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": workload_config(sv, per_rank),
             "engine": {"path": "whole time loops, one cooperative launch per group of shots"
-                       if q["kernel"] == "resident" else "batched, CUDA graph", "kernel": q["kernel"], "shots_per_launch": q["shots_per_batch"],
-                       "block_x": q["block_x"], "graph_branches": q["graph_branches"], "adjoint": args.adjoint,
+                       if q["kernel"] == "resident" else "batched, CUDA graph", "kernel": q["kernel"],
+                       "shots_per_launch": loops["reverse"]["shots"], "block_x": q["block_x"],
+                       "graph_branches": loops["reverse"]["branches"], "loops": loops, "adjoint": args.adjoint,
                        "parallelism": "shots" + ("" if world == 1 else " x%d ranks" % world)},
             "autotune": {"trial_steps": 48, "candidates": tuned} if tuned else None,
             "gpts_per_s": value * U / 1e9,
@@ -521,19 +523,23 @@ def run_mine(args):
         # the loop's batches and branches), the L2 roof, and the dominant kernel against both roofs
         prof = eng.profile_kernels()
         kb = kernel_bytes_per_shot(sv.nx, sv.nz, sv.npml, sv.ng, sv.nt)
-        nbatch = -(-per_rank // q["shots_per_batch"])
-        shots_launch = per_rank / nbatch  # mean shots per launch (the last batch may be smaller)
         vec, res = q["kernel"] == "vec", q["kernel"] == "resident"
         kern = {}
         for k, v in prof.items():
-            per_step = v["mean_ms"] * (nbatch if vec else v["launches"] / (sv.nt - 1))
+            # launches per time step; the vec kernels are replayed for at most 256 steps
+            per_step = v["mean_ms"] * v["launches"] / (min(sv.nt - 1, 256) if vec else sv.nt - 1)
             kern[k] = dict(v, ms_per_time_step=per_step, ms_per_gradient=per_step * (sv.nt - 1))
         tot = sum(x["ms_per_gradient"] for x in kern.values())
         for k in kern:
             kern[k]["share"] = kern[k]["ms_per_gradient"] / tot
         top = max(kern, key=lambda k: kern[k]["ms_per_gradient"])
+        # mean shots per launch (the last batch may be smaller)
         if res:
             shots_launch = per_rank / prof[top]["launches"]
+        elif vec:
+            shots_launch = per_rank / (prof[top]["launches"] / min(sv.nt - 1, 256))
+        else:
+            shots_launch = per_rank / -(-per_rank // q["shots_per_batch"])
         alg = kb[top] * shots_launch
         achieved = alg / (prof[top]["mean_ms"] / 1000.0) / 1e9
         l2 = l2_bandwidth()
@@ -550,7 +556,8 @@ def run_mine(args):
                             "algorithmic_bytes_per_launch": alg, "mean_launch_ms": prof[top]["mean_ms"],
                             "shots_per_launch": shots_launch,
                             "timing": ("each kernel alone in a CUDA graph of every batch on the loop's %d branches, "
-                                       "events around one replay" % q["graph_branches"]) if vec else
+                                       "events around one replay"
+                                       % loops["reverse" if top.startswith("bwd") else "saving"]["branches"]) if vec else
                                       "events around every launch",
                             "kernels": kern, "kernels_ms_per_gradient": tot,
                             "ms_per_step": ms_per_step}
@@ -797,8 +804,7 @@ def run_correlation(args):
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": sv.name, "grid": [sv.nx, sv.nz], "npml": sv.npml, "nt": sv.nt, "shots": sv.ns,
                        "receivers": sv.ng, "dx_m": sv.dx, "dt_s": sv.dt, "adjoint": args.adjoint,
-                       "kernel": q["kernel"], "shots_per_launch": q["shots_per_batch"],
-                       "graph_branches": q["graph_branches"],
+                       "kernel": q["kernel"], "loops": {k: eng.query_loop(k) for k in ("saving", "reverse")},
                        "memory": {"strategy": "checkpoints every %d steps" % ckpt if ckpt else "stored per step",
                                   "device_bytes": q["device_bytes"]},
                        "l2": "inputs larger than L2: each step streams the per-step records of every shot",

@@ -85,7 +85,8 @@ typedef struct swit_desc {
   int32_t kernel_variant;   /* 0 = automatic: FP32 engines on the batched path with
                                default launch shapes run whole time loops with
                                the wavefields in registers where the shots fit
-                               the device (swit_query reports 7 when both loops
+                               the device and that is estimated faster, each
+                               loop by itself (swit_query reports 7 when both
                                do), else vec; 1 = split: two kernels per step,
                                in place, one point per thread; 2 = walk: one
                                kernel per step, double-buffered, each warp
@@ -210,8 +211,9 @@ int swit_l2_bandwidth(int64_t bytes, int32_t reps, double* gbs, void* stream);
  * forward and reverse loop with an event pair around it.  With the walk
  * variant, [0] is the forward step kernel, [2] the reverse step kernel and [1],
  * [3] are unused (0 launches); with resident loops likewise, [0] being a forward
- * and [2] a reverse time loop of a group of shots.  Leaves the wavefields undefined until the next
- * forward run; synchronises the stream. */
+ * and [2] a reverse time loop of a group of shots (an engine with only one of
+ * these loops resident is timed on the step kernels).  Leaves the wavefields
+ * undefined until the next forward run; synchronises the stream. */
 int swit_profile_kernels(swit_engine* e, int32_t launches[4], double mean_ms[4], void* stream);
 
 /* Capacity of swit_forward_shot_static's fixed scratch (about 2.7 MB per GPU). */
@@ -244,8 +246,11 @@ int swit_forward_shot_static(int32_t nx, int32_t nz, int32_t npml, int32_t nt, f
                              const float* rec_z, const float* vp, const float* rho, const float* src, float* seis,
                              void* stream);
 
-/* Sizes and launch configuration the engine has chosen (graph_branches: the
- * concurrent branches its graphs use); any pointer may be NULL. */
+/* Sizes and launch configuration the engine has chosen.  shots_per_batch, block_x
+ * and graph_branches (the concurrent branches of its graphs) are those of the step
+ * kernels' reverse loop, also where the engine does not run it: kernel_variant is
+ * 7 when the saving forward and the reverse loop both run resident.
+ * swit_query_loop tells what each loop runs.  Any pointer may be NULL. */
 int swit_query(const swit_engine* e, int64_t* device_bytes, int32_t* shots_per_batch, int32_t* block_x,
                int32_t* kernels_per_forward, int32_t* kernels_per_backward, int32_t* kernel_variant,
                int32_t* graph_branches);

@@ -35,6 +35,18 @@ def test_branches(opts, shape, forward, reverse):
         assert e.query()["graph_branches"] == reverse
 
 
+@pytest.mark.parametrize("shape,kernel", [((481, 141, 40, 30), "resident"), ((587, 238, 48, 23), "vec")])
+def test_launch_counts_are_those_of_the_loops_that_run(shape, kernel):
+    s, _, _ = problem(*shape, nt=400)
+    with Engine(**s.engine_args()) as e:
+        q, rev, sav = e.query(), e.query_loop("reverse"), e.query_loop("saving")
+    assert q["kernel"] == rev["kernel"] == kernel and sav["kernel"] == "resident"
+    assert rev["branches"] == (1 if kernel == "resident" else 3)
+    per_launch = 1 if kernel == "resident" else 2 * (s.nt - 1)
+    assert q["kernels_per_backward"] == per_launch * -(-s.ns // rev["shots"])
+    assert q["kernels_per_forward"] == -(-s.ns // sav["shots"])
+
+
 def test_loops_on_different_branches_match_one_branch():
     s, src, rho = problem(1460, 716, 50, 4, 9)
     adj = np.random.default_rng(1).standard_normal((s.ns, s.ng, s.nt)).astype(np.float32)
