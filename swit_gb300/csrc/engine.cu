@@ -141,9 +141,9 @@ struct swit_engine {
   void *xm = nullptr, *xsrc = nullptr, *xdadc = nullptr;
   std::vector<cudaGraphExec_t> gxb;
   size_t graph_nodes = 0;  // node bound per captured graph (kGraphNodes; SWIT_GRAPH_NODES overrides)
-  // resident time loops (kernels_resident.cuh), where a split fits the device and is faster (ResLoop::alone); else
-  // the variant's kernels: forward (0) and saving forward (1), reverse, exact adjoint's reverse.  An instance of a
-  // multi-instance engine keeps every loop that fits
+  // resident time loops (kernels_resident.cuh) where a split fits the device: forward (0) and saving forward (1),
+  // reverse, exact adjoint's reverse.  The engine by itself runs those that are faster (ResLoop::alone), else the
+  // variant's kernels
   ResLoop *resf[2] = {nullptr, nullptr}, *resb = nullptr, *resx = nullptr;
   uint4* d_halo = nullptr;  // a launch's halo packets, then its stop word
   int wait_err = 0;         // error word that a call has reported and swit_check has not
@@ -699,6 +699,13 @@ inline bool caller_capturing(cudaStream_t st) {
   return cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusActive;
 }
 
+// The resident loop of a call: the faster one, or, while the caller captures a loop whose step kernels would be
+// too many nodes for one graph, any that fits.
+inline const ResLoop* res_for(const swit_engine* e, const ResLoop* l, int nbatch, cudaStream_t st) {
+  if (!l || l->alone) return l;
+  return (size_t)nbatch * loop_nodes(e) > e->graph_nodes && caller_capturing(st) ? l : nullptr;
+}
+
 template <class F>
 int issue_into_capture(swit_engine* e, cudaStream_t st, int branches, int nbatch, F&& issue) {
   // the caller's graph gets every node of the loop: keep it under the same bound
@@ -729,7 +736,8 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  if (res_alone(e->resf[store && !e->ckpt_k])) {
+  const int fb = fwd_batch(e), nbatch = (e->ns + fb - 1) / fb;
+  if (res_for(e, e->resf[store && !e->ckpt_k], nbatch, st)) {
     if (store && e->ckpt_k)
       forward_checkpointed<R>(e, 0, e->ns, st, true);
     else
@@ -738,7 +746,6 @@ int run_forward_loop(swit_engine* e, bool store, cudaStream_t st) {
     return 0;
   }
   std::vector<cudaGraphExec_t>& ex = e->gfwd[store ? 1 : 0];
-  const int fb = fwd_batch(e), nbatch = (e->ns + fb - 1) / fb;
   auto issue = [&](int b, cudaStream_t cs) {
     const int s0 = b * fb, nb = std::min(fb, e->ns - s0);
     if (store && e->ckpt_k)
@@ -766,7 +773,8 @@ int run_backward_loop(swit_engine* e, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  if (res_alone(e->resb)) {
+  const int nbatch = (e->ns + e->batch - 1) / e->batch;
+  if (res_for(e, e->ckpt_k && !e->resf[1] ? nullptr : e->resb, nbatch, st)) {
     if (e->ckpt_k)
       backward_checkpointed<R>(e, 0, e->ns, st, true);
     else
@@ -774,7 +782,6 @@ int run_backward_loop(swit_engine* e, cudaStream_t st) {
     CK(cudaGetLastError());
     return 0;
   }
-  const int nbatch = (e->ns + e->batch - 1) / e->batch;
   auto issue = [&](int b, cudaStream_t cs) {
     const int s0 = b * e->batch, nb = std::min(e->batch, e->ns - s0);
     if (e->ckpt_k)
@@ -2190,7 +2197,7 @@ static int res_setup(swit_engine* e, const swit_desc* d, bool multi) {
     }
     for (const auto& l : loops) {
       l.second->alone = ok && (forced || res < vec);
-      l.second->ok = l.second->alone || (multi && l.second->ok);
+      if (e->exact && !l.second->alone) l.second->ok = false;  // D has one layout
     }
   };
   keep({{kResLoopFwd, &f}});

@@ -181,3 +181,36 @@ def test_checkpointed_forward_and_reverse_on_different_kernels_match_the_step_ke
             out.append((e.forward(src, save_boundary=True), *e.backward(adj)))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("every", [0, 30])
+def test_capture_beyond_the_node_bound_takes_the_resident_loops_that_fit(every, monkeypatch):
+    """The reverse loop (with checkpoints also the forward) runs on the step kernels here; captured into a graph it
+    would exceed the bound, and the same results come from resident loops."""
+    import torch
+    s, src, rho = problem(338, 311, 51, 14, 90)
+    monkeypatch.setenv("SWIT_GRAPH_NODES", "300")
+    src = torch.from_numpy(src).cuda()
+    adj = torch.randn(s.ns, s.ng, s.nt, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    with Engine(**s.engine_args(), checkpoint_every=every) as e:
+        assert e.query_loop("reverse")["kernel"] == "vec"
+        e.set_model(s.vp_true, rho)
+        seis = torch.zeros(s.ns, s.ng, s.nt, device="cuda")
+        outs = [torch.zeros(s.nx, s.nz, device="cuda") for _ in range(3)]
+
+        def step():
+            e.forward(src, save_boundary=True, seis=seis)
+            e.backward(adj, *outs)
+        step()
+        torch.cuda.synchronize()
+        want = [x.clone() for x in (seis, *outs)]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+            step()
+        for x in (seis, *outs):
+            x.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        e.check()
+    for a, b in zip((seis, *outs), want):
+        torch.testing.assert_close(a, b, rtol=0, atol=0)
