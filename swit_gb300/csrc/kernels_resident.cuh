@@ -1047,7 +1047,7 @@ __device__ __forceinline__ void side_insert(const Tile<TX>& T, const ResPlan& r,
 // Five 16-value arrays and the rest need more registers than 128: 384 threads of 168 are faster on a full
 // device than 512 of 128, which spill (49 shots 481x141: 3.1 against 4.4 us per step and launch, 13 and 10
 // launches, before later steps).  Measured against the vec kernels: reverse step of 49 shots 481x141
-// 59.8 -> 35.5 us, of 5 shots 201x101 11.2 -> 2.4 us.
+// 59.8 -> 34.1 us, of 5 shots 201x101 11.2 -> 2.4 us.
 template <int TX, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
     k_bwd_res(const __grid_constant__ Grid<float> g, const __grid_constant__ ResPlan r,
